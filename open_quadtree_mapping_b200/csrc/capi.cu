@@ -154,12 +154,13 @@ void run_stage(const qm::JobDesc &J, const qm_params &p, const qm::Shape &s, con
 }
 
 // Workspace of the soft BP: the BP workspace of qm_bp_extract (pyramid data
-// and messages of every level), the message states of one level's half-sweeps
-// for the adjoint (sized for the largest level: iterations + 1 states), and
-// two adjoint buffers of the level-0 size.
+// and messages of every level), the message states that the forward's
+// half-sweeps leave for the adjoint (qm::HistLevel), and two adjoint buffers
+// of the level-0 size.
 struct SoftLayout
 {
   size_t bp = 0, hist = 0, dir = 0, total = 0;
+  size_t hist_off[qm::kMaxLevels] = {}; // from the end of bp
 };
 
 SoftLayout soft_layout(int W, int H, const qm_params &p)
@@ -171,7 +172,8 @@ SoftLayout soft_layout(int W, int H, const qm_params &p)
   for (int l = 0; l < p.bp_levels; ++l)
   {
     const size_t n = align256((size_t)w * h * p.num_hyp * sizeof(float));
-    L.hist = std::max(L.hist, (size_t)(p.bp_iters[l] + 1) * 4 * n);
+    L.hist_off[l] = L.hist;
+    L.hist += (size_t)qm::HistLevel::states(p.bp_iters[l]) * 4 * n;
     w = (w + 1) / 2;
     h = (h + 1) / 2;
   }
@@ -257,72 +259,109 @@ struct SoftBp
     return p;
   }
 
-  // Reverse mode over the whole pyramid, fine to coarse: the readout's
-  // adjoint enters at level 0; every level recomputes its half-sweeps from
-  // its starting state (all cells inherit the parents' final messages),
-  // keeping each state, then runs the half-sweep adjoints backwards and hands
-  // the adjoint of its starting state to the parents.
-  void backward(const qm_params &q, float tau, const float *g_sparse, double *gP,
-                cudaStream_t s)
+  qm::HistLevel hist_level(int l) const
+  {
+    const size_t n =
+        align256((size_t)J.lv[l].w * J.lv[l].h * J.D * sizeof(float)) / sizeof(float);
+    return qm::HistLevel{(float *)(hist + lay.hist_off[l]), n, 4 * n};
+  }
+
+  // Hierarchical BP with every half-sweep writing the state its adjoint will
+  // read (same bytes as in place, no copies), then the soft readout.  The
+  // coarse levels run as one cluster launch, as in the plain pipeline.
+  void forward(const qm_params &q, float tau, float *sparse, cudaStream_t s)
   {
     const int L = q.bp_levels, D = q.num_hyp;
     const qm::KParams kp = qm::kparams(q);
+    const qm::Batch B = qm::stage::single(J);
+    for (int l = 1; l < L; ++l)
+      qm::launch_pyramid(B, cdiv_i((long)J.lv[l].w * J.lv[l].h * (D / 4), qm::kFlatThreads), l, s);
+    int lc = L;
+    while (lc > 0 && q.bp_iters[lc - 1] >= 2 &&
+           (long)J.lv[lc - 1].w * J.lv[lc - 1].h <= QM_DEFAULT_COARSE_CELLS)
+      --lc;
+    if (lc < L)
+    {
+      qm::CoarsePlan cp;
+      std::memset(&cp, 0, sizeof(cp));
+      cp.lo = lc;
+      cp.hi = L - 1;
+      cp.keep = 1;
+      for (int l = 0; l < L; ++l)
+      {
+        cp.iters[l] = q.bp_iters[l];
+        cp.hist[l] = hist_level(l);
+      }
+      qm::launch_bp_coarse(B, 0, 1, D, cp, kp, q.arith, s);
+    }
+    for (int l = lc - 1; l >= 0; --l)
+    {
+      const qm::LevelDesc &V = J.lv[l];
+      const int iters = q.bp_iters[l];
+      if (iters < 2) // cells no half-sweep writes
+        qm::launch_msg_inherit(B, cdiv_i((long)V.w * V.h * (D / 4), qm::kFlatThreads), l, iters,
+                               q.qt_max_level, s);
+      const qm::HistLevel hl = hist_level(l);
+      for (int it = 0; it < iters; ++it)
+      {
+        qm::SweepIO io;
+        for (int m = 0; m < 4; ++m)
+        {
+          io.in[m] = it > 0 ? hl.at(it - 1, iters, m, V.msg[m]) : V.msg[m];
+          io.out[m] = hl.at(it, iters, m, V.msg[m]);
+        }
+        qm::launch_bp_sweep_io(B, D, l, it, io, kp, q.arith, s);
+      }
+    }
+    qm::check(cudaMemsetAsync(sparse, 0, sizeof(float) * J.W * J.H, s), "memset");
+    qm::DiffBp a = level_args(0, q, tau);
+    a.sparse = sparse;
+    qm::launch_soft_readout(a, 0, s);
+    qm::check(cudaGetLastError(), "soft BP");
+  }
+
+  // Reverse mode over the whole pyramid, fine to coarse: the readout's
+  // adjoint enters at level 0; every level runs its half-sweeps' adjoints
+  // backwards over the states the forward left and hands the adjoint of its
+  // starting state to the parents.
+  void backward(const qm_params &q, float tau, const float *g_sparse, double *gP,
+                cudaStream_t s)
+  {
+    const int L = q.bp_levels;
     qm::check(cudaMemsetAsync(gP, 0, 2 * sizeof(double), s), "memset");
     int cur = 0;
-    qm::check(cudaMemsetAsync(adj[cur], 0, 4 * lay.dir, s), "memset");
-    {
-      qm::DiffBp a = level_args(0, q, tau);
-      const qm::MsgPtrs A = adjoint(cur);
+    auto with = [&](qm::DiffBp a, const qm::MsgPtrs &A) {
       for (int m = 0; m < 4; ++m)
         a.A[m] = A.m[m];
+      return a;
+    };
+    {
+      qm::DiffBp a = with(level_args(0, q, tau), adjoint(cur));
       a.g_sparse = g_sparse;
       qm::launch_soft_readout(a, 1, s);
     }
-    const qm::Batch B = qm::stage::single(J);
     for (int l = 0; l < L; ++l)
     {
-      const int w = J.lv[l].w, h = J.lv[l].h;
-      const size_t n = (size_t)w * h * D;
-      const size_t slot = align256(n * sizeof(float));
-      auto state = [&](int i, int m) { return (float *)(hist + ((size_t)i * 4 + m) * slot); };
-      auto snapshot = [&](int i) {
-        for (int m = 0; m < 4; ++m)
-          qm::check(cudaMemcpyAsync(state(i, m), J.lv[l].msg[m], n * sizeof(float),
-                                    cudaMemcpyDeviceToDevice, s),
-                    "message snapshot");
-      };
-      qm::launch_msg_inherit(B, cdiv_i((long)w * h * (D / 4), qm::kFlatThreads), l, 0,
-                             q.qt_max_level, s);
-      snapshot(0);
-      const int sweep_blocks =
-          cdiv_i((long)((w + 1) / 2) * h, qm::kCellWarps * qm::bp_cells_per_warp(D));
-      const int it = q.bp_iters[l];
-      for (int i = 0; i < it; ++i)
+      const qm::LevelDesc &V = J.lv[l];
+      const qm::HistLevel hl = hist_level(l);
+      const int iters = q.bp_iters[l];
+      qm::DiffBp a = with(level_args(l, q, tau), adjoint(cur));
+      a.iters = iters;
+      a.gP = gP;
+      for (int i = iters - 1; i >= 0; --i)
       {
-        qm::launch_bp_sweep_own(B, sweep_blocks, D, l, i & 1, kp, q.arith, s);
-        snapshot(i + 1);
-      }
-      const qm::MsgPtrs A = adjoint(cur);
-      for (int i = it - 1; i >= 0; --i)
-      {
-        qm::DiffBp a = level_args(l, q, tau);
-        for (int m = 0; m < 4; ++m)
-        {
-          a.S[m] = state(i, m);
-          a.A[m] = A.m[m];
-        }
         a.parity = i & 1;
-        a.gP = gP;
+        a.last = i == iters - 1;
+        a.first = i == 0;
+        const bool top = l + 1 >= L;
+        a.pw = top ? 0 : J.lv[l + 1].w;
+        for (int m = 0; m < 4; ++m)
+          a.S[m] = i > 0 ? hl.at(i - 1, iters, m, V.msg[m]) : top ? nullptr : J.lv[l + 1].msg[m];
         qm::launch_bp_sweep_bwd(a, s);
       }
       if (l + 1 < L)
       {
-        const int pw = J.lv[l + 1].w, ph = J.lv[l + 1].h;
-        const qm::MsgPtrs P = adjoint(cur ^ 1);
-        for (int m = 0; m < 4; ++m)
-          qm::check(cudaMemsetAsync(P.m[m], 0, (size_t)pw * ph * D * sizeof(float), s),
-                    "memset");
-        qm::launch_msg_downsample_add(A, w, h, P, pw, ph, D, s);
+        qm::launch_msg_downsample(a, adjoint(cur ^ 1), J.lv[l + 1].w, J.lv[l + 1].h, s);
         cur ^= 1;
       }
     }
@@ -469,7 +508,6 @@ struct SoftBp64
   {
     qm::check(cudaMemsetAsync(gP, 0, 2 * sizeof(double), s), "memset");
     int cur = 0;
-    qm::check(cudaMemsetAsync(adj[cur], 0, 4 * lay.dir, s), "memset");
     {
       qm::DiffBp64 a = level_args(0, q, tau);
       const qm::MsgPtrs64 A = adjoint(cur);
@@ -492,26 +530,22 @@ struct SoftBp64
                   },
                   s);
       const qm::MsgPtrs64 A = adjoint(cur);
+      qm::DiffBp64 a = level_args(l, q, tau);
+      a.iters = q.bp_iters[l];
+      a.gP = gP;
+      for (int m = 0; m < 4; ++m)
+        a.A[m] = A.m[m];
       for (int i = q.bp_iters[l] - 1; i >= 0; --i)
       {
-        qm::DiffBp64 a = level_args(l, q, tau);
         for (int m = 0; m < 4; ++m)
-        {
           a.S[m] = state(i, m);
-          a.A[m] = A.m[m];
-        }
         a.parity = i & 1;
-        a.gP = gP;
+        a.last = i == q.bp_iters[l] - 1;
         qm::launch_bp_sweep_bwd(a, s);
       }
       if (l + 1 < L)
       {
-        const qm::MsgPtrs64 P = adjoint(cur ^ 1);
-        for (int m = 0; m < 4; ++m)
-          qm::check(cudaMemsetAsync(P.m[m], 0, (size_t)lw[l + 1] * lh[l + 1] * D * sizeof(double),
-                                    s),
-                    "memset");
-        qm::launch_msg_downsample_add(A, lw[l], lh[l], P, lw[l + 1], lh[l + 1], D, s);
+        qm::launch_msg_downsample(a, adjoint(cur ^ 1), lw[l + 1], lh[l + 1], s);
         cur ^= 1;
       }
     }
@@ -1282,15 +1316,7 @@ int qm_bp_soft_forward(const float *cost, int width, int height, const uint8_t *
     require(cost && levels && sparse && tau > 0.0f, "NULL argument or tau <= 0");
     const qm_params q = params_or_default(p);
     SoftBp sb(cost, width, height, levels, q, workspace, workspace_bytes);
-    const cudaStream_t s = as_stream(stream);
-    qm::check(cudaMemsetAsync(sparse, 0, sizeof(float) * width * height, s), "memset");
-    sb.J.sparse = sparse;
-    // hierarchical BP (its hard extraction is overwritten by the soft readout)
-    run_stage(sb.J, q, stage_shape(width, height, q, 1, nullptr), "bp", stream);
-    qm::DiffBp a = sb.level_args(0, q, tau);
-    a.sparse = sparse;
-    qm::launch_soft_readout(a, 0, s);
-    qm::check(cudaGetLastError(), "soft readout");
+    sb.forward(q, tau, sparse, as_stream(stream));
   });
 }
 

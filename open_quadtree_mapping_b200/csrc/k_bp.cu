@@ -24,6 +24,7 @@
 // Bytes per updated cell and half-sweep: 9*D*4 (data + 4 messages read, 4
 // messages written).
 #include <cfloat>
+#include <type_traits>
 
 #include "launch.h"
 
@@ -354,10 +355,14 @@ __device__ __forceinline__ void cell_update(const float (&dat)[HypLayout<D>::NV]
 }
 
 // One warp's lane groups of half-sweep `parity` at `level`: items item0 ..
-// item0 + G - 1 of the colour's cells (item = y * ceil(w / 2) + x / 2).
-template <int D, int ARITH, bool L2_ONLY>
+// item0 + G - 1 of the colour's cells (item = y * ceil(w / 2) + x / 2).  The
+// neighbours' messages come from the images in[4], the cells' own go to
+// out[4], by direction (both the level's own ones, except where the soft BP
+// keeps the states between half-sweeps).
+template <int D, int ARITH, bool L2_ONLY, class In, class Out>
 __device__ __forceinline__ void sweep_warp(const JobDesc &J, int level, int parity, int first,
-                                           int inherit, const KParams &kp, int item0)
+                                           int inherit, const KParams &kp, int item0, const In &in,
+                                           const Out &out_img)
 {
   using HL = HypLayout<D>;
   constexpr int NV = HL::NV, LPC = HL::LPC;
@@ -391,7 +396,7 @@ __device__ __forceinline__ void sweep_warp(const JobDesc &J, int level, int pari
       for (int k = 0; k < NV; ++k)
       {
         const int d = gl + LPC * k;
-        L.msg[m][c * D + d] = top ? 0.0f : msg_load<L2_ONLY>(C.msg[m] + pc + d);
+        out_img[m][c * D + d] = top ? 0.0f : msg_load<L2_ONLY>(C.msg[m] + pc + d);
       }
   }
   if (!__any_sync(0xffffffffu, act))
@@ -406,10 +411,10 @@ __device__ __forceinline__ void sweep_warp(const JobDesc &J, int level, int pari
   const float *src_u = nullptr, *src_d = nullptr, *src_l = nullptr, *src_r = nullptr;
   if (!first)
   {
-    src_u = L.msg[kDown] + (c - w) * D;
-    src_d = L.msg[kUp] + (c + w) * D;
-    src_l = L.msg[kRight] + (c - 1) * D;
-    src_r = L.msg[kLeft] + (c + 1) * D;
+    src_u = in[kDown] + (c - w) * D;
+    src_d = in[kUp] + (c + w) * D;
+    src_l = in[kRight] + (c - 1) * D;
+    src_r = in[kLeft] + (c + 1) * D;
   }
   else if (level + 1 < J.nlev)
   {
@@ -437,7 +442,7 @@ __device__ __forceinline__ void sweep_warp(const JobDesc &J, int level, int pari
                         [&](int dir, const float(&m)[NV], float mean) {
                           if (act)
                           {
-                            float *out = L.msg[dir] + c * D;
+                            float *out = out_img[dir] + c * D;
 #pragma unroll
                             for (int k = 0; k < NV; ++k)
                               out[gl + LPC * k] = m[k] - mean;
@@ -460,7 +465,23 @@ __global__ void __launch_bounds__(kMaxCellWarps * 32, 4)
   const int item0 = (lb * (int)(blockDim.x >> 5) + (threadIdx.x >> 5)) * G;
   if (item0 >= hw * L.h)
     return; // the whole warp
-  sweep_warp<D, ARITH, false>(J, level, parity, first, inherit, kp, item0);
+  sweep_warp<D, ARITH, false>(J, level, parity, first, inherit, kp, item0, L.msg, L.msg);
+}
+
+// Half-sweep `parity` from the message images io.in into io.out (the soft BP,
+// which keeps the states its adjoint reads): every cell of the colour is
+// written, those the quadtree test skips with their parents' messages.
+template <int D, int ARITH>
+__global__ void __launch_bounds__(kMaxCellWarps * 32, 4)
+    k_bp_sweep_io(const __grid_constant__ Batch B, int level, int parity, int first,
+                  const __grid_constant__ SweepIO io, KParams kp)
+{
+  constexpr int G = HypLayout<D>::G;
+  const LevelDesc &L = B.one.lv[level];
+  const int item0 = ((int)blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5)) * G;
+  if (item0 >= (L.w + 1) / 2 * L.h)
+    return; // the whole warp
+  sweep_warp<D, ARITH, false>(B.one, level, parity, first, 1, kp, item0, io.in, io.out);
 }
 
 // Every half-sweep of the coarse levels lo..hi (coarse to fine) in one
@@ -474,9 +495,13 @@ __global__ void __launch_bounds__(kMaxCellWarps * 32, 4)
 // the messages are bit-identical; messages are read through L2 because other
 // blocks of the cluster wrote them.  Every block of a cluster takes the same
 // barriers: the trip counts depend only on the job and the plan.
-template <int D, int ARITH>
+//
+// HIST: the half-sweeps read and write the plan's states (message_state), as
+// the adjoint of the soft BP needs them.
+template <int D, int ARITH, bool HIST>
 __global__ void __cluster_dims__(kCoarseCtas, 1, 1) __launch_bounds__(kCoarseThreads, 2)
-    k_bp_coarse(const __grid_constant__ Batch B, int j0, CoarsePlan plan, KParams kp)
+    k_bp_coarse(const __grid_constant__ Batch B, int j0, const __grid_constant__ CoarsePlan plan,
+                KParams kp)
 {
   constexpr int G = HypLayout<D>::G;
   const int job = j0 + (int)blockIdx.x / kCoarseCtas;
@@ -493,9 +518,22 @@ __global__ void __cluster_dims__(kCoarseCtas, 1, 1) __launch_bounds__(kCoarseThr
     const int iters = plan.iters[level];
     for (int it = 0; it < iters; ++it)
     {
-      for (int item0 = gw * G; item0 < n; item0 += stride)
-        sweep_warp<D, ARITH, true>(J, level, it & 1, it == 0 ? 1 : 0, it < 2 ? 1 : 0, kp,
-                                   item0);
+      if constexpr (HIST)
+      {
+        float *in[4], *out[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+        {
+          in[m] = plan.hist[level].at(it - 1, iters, m, L.msg[m]);
+          out[m] = plan.hist[level].at(it, iters, m, L.msg[m]);
+        }
+        for (int item0 = gw * G; item0 < n; item0 += stride)
+          sweep_warp<D, ARITH, true>(J, level, it & 1, it == 0 ? 1 : 0, 1, kp, item0, in, out);
+      }
+      else
+        for (int item0 = gw * G; item0 < n; item0 += stride)
+          sweep_warp<D, ARITH, true>(J, level, it & 1, it == 0 ? 1 : 0, it < 2 ? 1 : 0, kp, item0,
+                                     L.msg, L.msg);
       asm volatile("barrier.cluster.arrive.release.aligned;\n"
                    "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     }
@@ -621,15 +659,27 @@ void sweep_d(const Batch &B, int blocks, int level, int parity, int first, int i
         <<<blocks, warps * 32, 0, s>>>(B, level, parity, first, inherit, kp);
 }
 
-template <int D>
+template <int D, bool HIST>
 void coarse_d(const Batch &B, int j0, int jobs, const CoarsePlan &plan, KParams kp, int arith,
               cudaStream_t s)
 {
+  const int g = jobs * kCoarseCtas;
   if (arith == QM_ARITH_IEEE)
-    k_bp_coarse<D, QM_ARITH_IEEE><<<jobs * kCoarseCtas, kCoarseThreads, 0, s>>>(B, j0, plan, kp);
+    k_bp_coarse<D, QM_ARITH_IEEE, HIST><<<g, kCoarseThreads, 0, s>>>(B, j0, plan, kp);
   else
-    k_bp_coarse<D, QM_ARITH_REFERENCE>
-        <<<jobs * kCoarseCtas, kCoarseThreads, 0, s>>>(B, j0, plan, kp);
+    k_bp_coarse<D, QM_ARITH_REFERENCE, HIST><<<g, kCoarseThreads, 0, s>>>(B, j0, plan, kp);
+}
+
+template <int D>
+void sweep_io_d(const Batch &B, int blocks, int level, int it, const SweepIO &io, KParams kp,
+                int arith, cudaStream_t s)
+{
+  if (arith == QM_ARITH_IEEE)
+    k_bp_sweep_io<D, QM_ARITH_IEEE>
+        <<<blocks, kCellWarps * 32, 0, s>>>(B, level, it & 1, it == 0, io, kp);
+  else
+    k_bp_sweep_io<D, QM_ARITH_REFERENCE>
+        <<<blocks, kCellWarps * 32, 0, s>>>(B, level, it & 1, it == 0, io, kp);
 }
 
 template <int D>
@@ -641,6 +691,24 @@ void extract_d(const Batch &B, int blocks, int arith, int warps, cudaStream_t s)
     k_extract<D, QM_ARITH_REFERENCE><<<blocks, warps * 32, 0, s>>>(B);
 }
 
+} // namespace
+
+namespace
+{
+// f(std::integral_constant<int, d>) for a supported hypothesis count
+template <class F>
+void by_d(int d, F &&f)
+{
+  switch (d)
+  {
+  case 32: f(std::integral_constant<int, 32>()); break;
+  case 48: f(std::integral_constant<int, 48>()); break;
+  case 64: f(std::integral_constant<int, 64>()); break;
+  case 96: f(std::integral_constant<int, 96>()); break;
+  case 128: f(std::integral_constant<int, 128>()); break;
+  default: break;
+  }
+}
 } // namespace
 
 bool bp_supported_d(int d) { return d == 32 || d == 48 || d == 64 || d == 96 || d == 128; }
@@ -696,24 +764,27 @@ void launch_bp_sweep(const Batch &B, int blocks, int d, int level, int it, KPara
             warps, s);
 }
 
-void launch_bp_sweep_own(const Batch &B, int blocks, int d, int level, int parity, KParams kp,
-                         int arith, cudaStream_t s, int warps)
+void launch_bp_sweep_io(const Batch &B, int d, int level, int it, const SweepIO &io, KParams kp,
+                        int arith, cudaStream_t s)
 {
-  sweep_any(B, blocks, d, level, parity, 0, 0, kp, arith, warps, s);
+  const LevelDesc &L = B.one.lv[level];
+  const int per = kCellWarps * bp_cells_per_warp(d);
+  const int blocks = ((L.w + 1) / 2 * L.h + per - 1) / per;
+  if (blocks > 0)
+    by_d(d, [&](auto dc) {
+      sweep_io_d<decltype(dc)::value>(B, blocks, level, it, io, kp, arith, s);
+    });
 }
 
 void launch_bp_coarse(const Batch &B, int j0, int jobs, int d, const CoarsePlan &plan,
                       KParams kp, int arith, cudaStream_t s)
 {
-  switch (d)
-  {
-  case 32: coarse_d<32>(B, j0, jobs, plan, kp, arith, s); break;
-  case 48: coarse_d<48>(B, j0, jobs, plan, kp, arith, s); break;
-  case 64: coarse_d<64>(B, j0, jobs, plan, kp, arith, s); break;
-  case 96: coarse_d<96>(B, j0, jobs, plan, kp, arith, s); break;
-  case 128: coarse_d<128>(B, j0, jobs, plan, kp, arith, s); break;
-  default: break;
-  }
+  by_d(d, [&](auto dc) {
+    if (plan.keep)
+      coarse_d<decltype(dc)::value, true>(B, j0, jobs, plan, kp, arith, s);
+    else
+      coarse_d<decltype(dc)::value, false>(B, j0, jobs, plan, kp, arith, s);
+  });
 }
 
 void launch_extract(const Batch &B, int blocks, int d, int arith, cudaStream_t s, int warps)

@@ -70,10 +70,32 @@ void launch_msg_inherit(const Batch &B, int blocks, int level, int iters, int qt
 // must have at least two half-sweeps)
 void launch_bp_sweep(const Batch &B, int blocks, int d, int level, int it, KParams kp, int arith,
                      cudaStream_t s, int warps = kCellWarps, int inherit = 0);
-// a half-sweep of colour `parity` that reads every incoming message from the
-// level's own buffers (all cells' starting messages already written)
-void launch_bp_sweep_own(const Batch &B, int blocks, int d, int level, int parity, KParams kp,
-                         int arith, cudaStream_t s, int warps = kCellWarps);
+// Message states a level keeps for the adjoint of the soft BP.  Half-sweeps
+// it = iters - 1 and iters - 2 write the level's own message images (together
+// every cell), the two before them the first kept state, and so on: half-sweep
+// it + 1 and its adjoint only read the colour that half-sweep it wrote.
+struct HistLevel
+{
+  float *base;      // kept states, 4 images each (null: none)
+  size_t dir, slot; // floats between the images of a state and between states
+  // image `m` of the state half-sweep `it` writes; own: the level's image
+  __host__ __device__ float *at(int it, int iters, int m, float *own) const
+  {
+    const int k = (iters - 1 - it) >> 1;
+    return k <= 0 ? own : base + (size_t)(k - 1) * slot + (size_t)m * dir;
+  }
+  __host__ __device__ static int states(int iters) { return iters > 2 ? (iters - 1) / 2 : 0; }
+};
+// message images a half-sweep reads and writes, by direction
+struct SweepIO
+{
+  const float *in[4];
+  float *out[4];
+};
+// half-sweep `it` of the inline job's level from io.in (it = 0: the parents'
+// messages) into io.out, skipped cells included
+void launch_bp_sweep_io(const Batch &B, int d, int level, int it, const SweepIO &io, KParams kp,
+                        int arith, cudaStream_t s);
 // Coarse BP levels in one launch (k_bp_coarse): levels hi down to lo, every
 // one with at least two half-sweeps (their first two write the inherited
 // messages), one cluster of kCoarseCtas blocks of kCoarseThreads threads per
@@ -84,6 +106,8 @@ struct CoarsePlan
 {
   int lo, hi;
   int iters[kMaxLevels];
+  int keep; // 1: the half-sweeps keep their states in hist
+  HistLevel hist[kMaxLevels];
 };
 void launch_bp_coarse(const Batch &B, int j0, int jobs, int d, const CoarsePlan &plan,
                       KParams kp, int arith, cudaStream_t s);
@@ -125,9 +149,13 @@ struct DiffBpR
   int W, H, D;           // image and hypotheses
   int w, h;              // cells of this level
   int level, parity, qt_max;
+  int first;             // half-sweep 0: S holds the parents' messages, pw wide
+                         // (null at the coarsest level: zeros)
+  int last;              // the level's last half-sweep (adjoint: the first)
+  int iters, pw;
   const uint8_t *levels; // quadtree level map
   const R *data;         // data term of this level
-  const R *S[4];         // messages read (a state snapshot, or the finals)
+  const R *S[4];         // messages read (a kept state, or the finals)
   R *A[4];               // adjoint of the messages, by direction
   float P1, P2;
   double *gP;            // dL/dP1, dL/dP2 (accumulated)
@@ -145,20 +173,24 @@ struct MsgPtrsR
 };
 using MsgPtrs = MsgPtrsR<float>;
 using MsgPtrs64 = MsgPtrsR<double>;
-// soft readout at level-0 node cells: forward writes sparse; backward adds
-// the belief adjoint to A (the four incoming messages of every node cell)
+// soft readout at level-0 node cells: forward writes sparse; backward writes
+// every value of A, the belief adjoint at the four incoming messages of every
+// node cell and 0 elsewhere
 void launch_soft_readout(const DiffBp &a, int backward, cudaStream_t s);
 void launch_soft_readout(const DiffBp64 &a, int backward, cudaStream_t s);
-// adjoint of one half-sweep of colour a.parity: reads A at the updated cells
-// (then zeroes it) and adds to A at the messages they read (a.S is the state
-// the forward half-sweep read)
+// adjoint of one half-sweep of colour a.parity: consumes A at the updated
+// cells and writes the adjoints of the messages they read (a.S, the state the
+// forward half-sweep read).  Values of A it has consumed are left stale; they
+// are rewritten before they are read again, and launch_msg_downsample skips
+// those of the colour of half-sweep 0.
 void launch_bp_sweep_bwd(const DiffBp &a, cudaStream_t s);
 void launch_bp_sweep_bwd(const DiffBp64 &a, cudaStream_t s);
-// parent.m[k] += sum of the (up to four) children's child.m[k], k = 0..3
-void launch_msg_downsample_add(const MsgPtrs &child, int cw, int ch, const MsgPtrs &parent,
-                               int pw, int ph, int D, cudaStream_t s);
-void launch_msg_downsample_add(const MsgPtrs64 &child, int cw, int ch, const MsgPtrs64 &parent,
-                               int pw, int ph, int D, cudaStream_t s);
+// parent.m[k] = sum of the (up to four) children's adjoints a.A[k] of the
+// starting messages of level a (pw x ph parents)
+void launch_msg_downsample(const DiffBp &a, const MsgPtrs &parent, int pw, int ph,
+                           cudaStream_t s);
+void launch_msg_downsample(const DiffBp64 &a, const MsgPtrs64 &parent, int pw, int ph,
+                           cudaStream_t s);
 // FP64 BP forward of the gradient-check mode (the product's BP is FP32):
 // out[i] = in[i] widened; the pyramid of data terms (children summed x
 // offset outer, y offset inner); every cell of a level starting from its
