@@ -397,10 +397,10 @@ int qm_semidense_step(const uint8_t *key, const uint8_t *inc, int width, int hei
  * readout at the node cells: p(d) = softmax(-belief(d) / tau), depth =
  * 1 / (inv_depth_step * sum p(d) d + min_inv_depth), written at (4x, 4y) of
  * every node cell of `sparse` (zero elsewhere).  qm_bp_soft_backward takes
- * the same inputs, the workspace as the forward left it, and dL/d sparse,
- * and writes dL/dP1, dL/dP2 to grad_penalties (2 device doubles); it
- * recomputes the messages of each level instead of storing all of them.
- * cost and workspace 16-byte aligned. */
+ * the same inputs, the workspace as the forward left it (with the message
+ * states the adjoint reads; it may run more than once over them), and
+ * dL/d sparse, and writes dL/dP1, dL/dP2 to grad_penalties (2 device
+ * doubles).  cost and workspace 16-byte aligned. */
 int qm_bp_soft_workspace_size(int width, int height, const qm_params *p, size_t *bytes);
 int qm_bp_soft_forward(const float *cost, int width, int height, const uint8_t *levels,
                        const qm_params *p, float tau, float *sparse, void *workspace,

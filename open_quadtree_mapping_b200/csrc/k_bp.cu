@@ -8,15 +8,13 @@
 // Jacobi step inside the colour, exactly as the reference's launch.
 //
 // Lane groups: a cell is handled by a group of LPC lanes (32 for 96 and 128
-// hypotheses, 16 for 48 and 64, 8 for 32), so a warp updates 32/LPC cells
-// at once; lane g of a group holds hypotheses g, g+LPC, g+2*LPC, ... (3 or
-// 4 register slots; every supported count is exactly LPC x slots).  The four
-// directions are computed from one load of the data cost and the four
-// incoming messages.  The normalising sum uses the reference's stride-halving
-// tree (bpextract.cu:293-300) over the next power of two P >= D with zero
-// padding: strides >= LPC combine register slots, strides < LPC run as an
-// xor butterfly inside the group, so lane 0 of the group ends with the
-// bit-identical sum (and, addition being commutative, so does every lane).
+// hypotheses, 16 for 48 and 64, 8 for 32), so a warp updates 32/LPC cells at
+// once.  The half-sweeps hold four consecutive hypotheses per lane
+// (QuadLayout), the extraction the hypotheses g, g+LPC, g+2*LPC, ... in lane g
+// (HypLayout; every supported count is exactly LPC x 3 or 4).  The four
+// directions are computed from one load of the data cost and the four incoming
+// messages.  The normalising sum uses the reference's stride-halving tree
+// (bpextract.cu:293-300) over the next power of two P >= D with zero padding.
 // The argmin of the extraction uses the same tree with the reference's tie
 // rule (the right element wins only when strictly smaller,
 // bpextract.cu:347-355).
@@ -51,67 +49,6 @@ struct HypLayout
   static constexpr int G = 32 / LPC;                  // cells per warp
   static_assert(NV * LPC == D, "hypothesis count must fill the lane group");
 };
-
-// Stride-halving tree sum over the D values of a lane group, held as
-// v[k] = value(g + LPC*k).  Strides >= LPC combine register slots (the
-// padding beyond D is zero, so those additions are skipped); strides < LPC
-// run as an xor butterfly inside the group.  Lane 0 of the group performs
-// exactly the reference's additions, and since a + b == b + a bit for bit,
-// every lane of the group ends with lane 0's value.
-template <int D>
-__device__ __forceinline__ float tree_sum(const float (&v)[HypLayout<D>::NV])
-{
-  constexpr int P = HypLayout<D>::P;
-  constexpr int NV = HypLayout<D>::NV;
-  constexpr int LPC = HypLayout<D>::LPC;
-  float a[NV];
-#pragma unroll
-  for (int k = 0; k < NV; ++k)
-    a[k] = v[k];
-#pragma unroll
-  for (int s = P / 2; s >= LPC; s /= 2)
-  {
-    const int t = s / LPC;
-#pragma unroll
-    for (int k = 0; k < t; ++k)
-      if (k + t < NV)
-        a[k] += a[k + t];
-  }
-  float r = a[0];
-#pragma unroll
-  for (int o = LPC / 2; o > 0; o >>= 1)
-    r += __shfl_xor_sync(0xffffffffu, r, o);
-  return r;
-}
-
-// Order-preserving map between floats and signed ints (an involution), so a
-// float minimum can use the integer warp reduction.
-__device__ __forceinline__ int order_key(float f)
-{
-  const int b = __float_as_int(f);
-  return b ^ ((b >> 31) & 0x7fffffff);
-}
-
-__device__ __forceinline__ float warp_min_redux(float v)
-{
-  const int k = __reduce_min_sync(0xffffffffu, order_key(v));
-  return __int_as_float(k ^ ((k >> 31) & 0x7fffffff));
-}
-
-// minimum over a lane group (exact, order-free)
-template <int LPC>
-__device__ __forceinline__ float group_min(float v)
-{
-  if constexpr (LPC == 32)
-    return warp_min_redux(v);
-  else
-  {
-#pragma unroll
-    for (int o = LPC / 2; o > 0; o >>= 1)
-      v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-  }
-}
 
 template <int D>
 __device__ __forceinline__ void tree_argmin(const float (&v)[HypLayout<D>::NV], int gl,
@@ -273,84 +210,178 @@ __global__ void __launch_bounds__(kFlatThreads)
 // kernel below, whose blocks hand messages to each other across cluster
 // barriers; the one-launch-per-half-sweep kernel reads them normally.
 template <bool L2_ONLY>
-__device__ __forceinline__ float msg_load(const float *p)
+__device__ __forceinline__ float4 msg_load(const float *p)
 {
   if constexpr (L2_ONLY)
-    return __ldcg(p);
+    return __ldcg(reinterpret_cast<const float4 *>(p));
   else
-    return *p;
+    return *reinterpret_cast<const float4 *>(p);
+}
+
+// ---- layout of the half-sweeps: lane g of a cell's group holds the four
+// consecutive hypotheses 4 g .. 4 g + 3 (one 16-byte load per message image
+// instead of four 4-byte ones; d +- 1 needs two shuffles per direction instead
+// of eight).  Groups have P / 4 lanes, as above; at 48 and 96 hypotheses the
+// last quarter of a group's lanes holds padding.
+template <int D>
+struct QuadLayout
+{
+  static constexpr int P = HypLayout<D>::P, LPC = P / 4, ACT = D / 4;
+  static_assert(LPC == HypLayout<D>::LPC, "one group layout");
+};
+
+// One reduction step across lanes gl and gl ^ o that also halves the values a
+// lane holds: lanes with bit o clear go on with lo, the others with hi.
+template <int N, class Op>
+__device__ __forceinline__ void halve(float (&lo)[N], const float (&hi)[N], bool up, int o, Op op)
+{
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+  {
+    const float send = up ? lo[i] : hi[i], keep = up ? hi[i] : lo[i];
+    lo[i] = op(keep, __shfl_xor_sync(0xffffffffu, send, o));
+  }
+}
+
+// v[dir] of the group from the lane that holds direction dir's result: the
+// directions are split over the two top bits of the lane's index in its group
+template <int LPC>
+__device__ __forceinline__ float from_dir(float r, int dir)
+{
+  return __shfl_sync(0xffffffffu, r, (dir >> 1) * (LPC / 2) + (dir & 1) * (LPC / 4), LPC);
+}
+
+// The group's minimum of v[dir] for the direction this lane holds.
+template <int LPC>
+__device__ __forceinline__ float dir_min(const float (&v)[4], int gl)
+{
+  auto mn = [](float a, float b) { return fminf(a, b); };
+  float a[2] = {v[0], v[1]}, b[2] = {v[2], v[3]};
+  halve(a, b, (gl & (LPC / 2)) != 0, LPC / 2, mn);
+  float c[1] = {a[0]}, d[1] = {a[1]};
+  halve(c, d, (gl & (LPC / 4)) != 0, LPC / 4, mn);
+  float r = c[0];
+#pragma unroll
+  for (int o = LPC / 8; o > 0; o >>= 1)
+    r = fminf(r, __shfl_xor_sync(0xffffffffu, r, o));
+  return r;
+}
+
+// The reference's stride-halving tree sum (bpextract.cu:293-300) of
+// m[dir][j] = value(4 g + j) over the group, for the direction this lane
+// holds.  Strides of four and more pair lanes: every step adds exactly the
+// tree's pairs (addition commutes bit for bit) while the lanes share out the
+// directions, then the four j; strides 2 and 1 pair the lanes that hold j and
+// j ^ 2, j ^ 1.  Padding is zero.
+template <int LPC>
+__device__ __forceinline__ float dir_tree_sum(const float (&m)[4][4], int gl)
+{
+  auto add = [](float a, float b) { return a + b; };
+  float a[8], b[8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+  {
+    a[j] = m[0][j], a[4 + j] = m[1][j];
+    b[j] = m[2][j], b[4 + j] = m[3][j];
+  }
+  halve(a, b, (gl & (LPC / 2)) != 0, LPC / 2, add);
+  float c[4] = {a[0], a[1], a[2], a[3]}, d[4] = {a[4], a[5], a[6], a[7]};
+  halve(c, d, (gl & (LPC / 4)) != 0, LPC / 4, add);
+  constexpr int o2 = LPC / 8, o1 = LPC / 16; // lane bits that share out j
+  float e[2] = {c[0], c[1]}, f[2] = {c[2], c[3]};
+  halve(e, f, (gl & o2) != 0, o2, add);
+  if constexpr (o1 == 0)
+  {
+    // eight lanes: the pair (j, j ^ 2) is in lanes gl, gl ^ 1, j and j ^ 1 here
+    const float s0 = e[0] + __shfl_xor_sync(0xffffffffu, e[0], o2);
+    const float s1 = e[1] + __shfl_xor_sync(0xffffffffu, e[1], o2);
+    return s0 + s1;
+  }
+  else
+  {
+    float r[1] = {e[0]}, q[1] = {e[1]};
+    halve(r, q, (gl & o1) != 0, o1, add);
+    float s = r[0];
+#pragma unroll
+    for (int o = o1 / 2; o > 0; o >>= 1)
+      s += __shfl_xor_sync(0xffffffffu, s, o);
+    s += __shfl_xor_sync(0xffffffffu, s, o2);
+    s += __shfl_xor_sync(0xffffffffu, s, o1);
+    return s;
+  }
 }
 
 // The update of one cell (bp, bpextract.cu:200-312) from its data term and
-// its four incoming messages (zeros, and has_* false, where the level ends),
-// every lane of the warp taking part (groups without a cell pass zeros):
-// for each outgoing direction, emit(dir, m, mean) receives the group's NV
-// values m[k] (hypothesis gl + LPC k) and the mean the message subtracts, so
-// the message is m[k] - mean.
+// its four incoming messages (zeros where the level ends: the reference leaves
+// those terms out, and adding 0 changes no value), every lane of the warp
+// taking part (groups without a cell pass zeros): for each outgoing direction,
+// emit(dir, v) receives the lane's four values of the message.
+// Padding lanes (gl >= ACT) pass anything.
 template <int D, int ARITH, class Emit>
-__device__ __forceinline__ void cell_update(const float (&dat)[HypLayout<D>::NV],
-                                            const float (&fu)[HypLayout<D>::NV],
-                                            const float (&fd)[HypLayout<D>::NV],
-                                            const float (&fl)[HypLayout<D>::NV],
-                                            const float (&fr)[HypLayout<D>::NV], bool has_u,
-                                            bool has_d, bool has_l, bool has_r, const KParams &kp,
+__device__ __forceinline__ void cell_update(const float4 &dat, const float4 &fu, const float4 &fd,
+                                            const float4 &fl, const float4 &fr, const KParams &kp,
                                             int gl, Emit &&emit)
 {
-  using HL = HypLayout<D>;
-  constexpr int NV = HL::NV, LPC = HL::LPC;
-  const float P1 = kp.P1, P2 = kp.P2;
+  constexpr int LPC = QuadLayout<D>::LPC, ACT = QuadLayout<D>::ACT;
+  const bool pad = ACT < LPC && gl >= ACT;
+  const float da[4] = {dat.x, dat.y, dat.z, dat.w}, ua[4] = {fu.x, fu.y, fu.z, fu.w};
+  const float ba[4] = {fd.x, fd.y, fd.z, fd.w}, la[4] = {fl.x, fl.y, fl.z, fl.w};
+  const float ra[4] = {fr.x, fr.y, fr.z, fr.w};
   // h of every direction: the data term plus the three other incoming
-  // messages, in the reference's order (up, down, left, right skipped as
-  // named by the direction); computed up front so the raw inputs die early
-  float hall[4][NV];
+  // messages, in the reference's order (up, down, left, right, the
+  // direction's own left out)
+  float h[4][4], low[4];
 #pragma unroll
-  for (int dir = 0; dir < 4; ++dir)
-#pragma unroll
-    for (int k = 0; k < NV; ++k)
-    {
-      float v = dat[k];
-      if (dir != kUp && has_u)
-        v += fu[k];
-      if (dir != kDown && has_d)
-        v += fd[k];
-      if (dir != kLeft && has_l)
-        v += fl[k];
-      if (dir != kRight && has_r)
-        v += fr[k];
-      hall[dir][k] = v;
-    }
+  for (int j = 0; j < 4; ++j)
+  {
+    const float du = da[j] + ua[j], dud = du + ba[j];
+    h[kUp][j] = ((da[j] + ba[j]) + la[j]) + ra[j];
+    h[kDown][j] = (du + la[j]) + ra[j];
+    h[kLeft][j] = dud + ra[j];
+    h[kRight][j] = dud + la[j];
+  }
 #pragma unroll
   for (int dir = 0; dir < 4; ++dir)
   {
-    const float(&hv)[NV] = hall[dir];
-    float lmin = FLT_MAX;
+    low[dir] = fminf(fminf(h[dir][0], h[dir][1]), fminf(h[dir][2], h[dir][3]));
+    if (pad)
+      low[dir] = FLT_MAX;
+  }
+  const float cap = dir_min<LPC>(low, gl) + kp.P2;
 #pragma unroll
-    for (int k = 0; k < NV; ++k)
-      lmin = fminf(lmin, hv[k]);
-    const float hmin = group_min<LPC>(lmin);
-    float m[NV];
+  for (int dir = 0; dir < 4; ++dir)
+  {
+    // the minimum over h(d), h(d - 1) + P1, h(d + 1) + P1, min h + P2
+    const float c = from_dir<LPC>(cap, dir);
+    float s[4];
 #pragma unroll
-    for (int k = 0; k < NV; ++k)
-    {
-      const int d = gl + LPC * k;
-      // h(d-1): the previous lane's slot k, or for group lane 0 the group's
-      // last lane's slot k-1; h(d+1): the next lane's slot k, or for the last
-      // lane group lane 0's slot k+1.  One shuffle each, the source lane
-      // choosing which register it offers.
-      const float up_src = (gl == LPC - 1 && k > 0) ? hv[k > 0 ? k - 1 : 0] : hv[k];
-      const float dn_src = (gl == 0 && k + 1 < NV) ? hv[k + 1 < NV ? k + 1 : k] : hv[k];
-      const float prev = __shfl_sync(0xffffffffu, up_src, (gl + LPC - 1) & (LPC - 1), LPC);
-      const float next = __shfl_sync(0xffffffffu, dn_src, (gl + 1) & (LPC - 1), LPC);
-      float mv = hv[k];
-      if (d > 0)
-        mv = fminf(mv, prev + P1);
-      if (d < D - 1)
-        mv = fminf(mv, next + P1);
-      m[k] = fminf(mv, hmin + P2);
-    }
-    const float sum = tree_sum<D>(m);
-    const float mean = mean_of<D, ARITH>(sum);
-    emit(dir, m, mean);
+    for (int j = 0; j < 4; ++j)
+      s[j] = h[dir][j] + kp.P1;
+    float prev = __shfl_up_sync(0xffffffffu, s[3], 1, LPC);
+    float next = __shfl_down_sync(0xffffffffu, s[0], 1, LPC);
+    if (gl == 0)
+      prev = c;
+    if (gl >= ACT - 1)
+      next = c;
+    h[dir][0] = fminf(fminf(h[dir][0], prev), fminf(s[1], c));
+    h[dir][1] = fminf(fminf(h[dir][1], s[0]), fminf(s[2], c));
+    h[dir][2] = fminf(fminf(h[dir][2], s[1]), fminf(s[3], c));
+    h[dir][3] = fminf(fminf(h[dir][3], s[2]), fminf(next, c));
+    if (pad)
+      h[dir][0] = h[dir][1] = h[dir][2] = h[dir][3] = 0.0f;
+  }
+  // in reference arithmetic the division by the constant count is left beside
+  // the subtraction, where the compiler may fuse the two (as it does in
+  // m - sum / DEPTH_NUM of one thread); IEEE divides once per direction
+  constexpr bool kIeee = ARITH == QM_ARITH_IEEE;
+  const float sum = dir_tree_sum<LPC>(h, gl);
+  const float mean = kIeee ? mean_of<D, ARITH>(sum) : sum;
+#pragma unroll
+  for (int dir = 0; dir < 4; ++dir)
+  {
+    const float got = from_dir<LPC>(mean, dir);
+    const float mu = kIeee ? got : mean_of<D, ARITH>(got);
+    emit(dir, make_float4(h[dir][0] - mu, h[dir][1] - mu, h[dir][2] - mu, h[dir][3] - mu));
   }
 }
 
@@ -364,11 +395,12 @@ __device__ __forceinline__ void sweep_warp(const JobDesc &J, int level, int pari
                                            int inherit, const KParams &kp, int item0, const In &in,
                                            const Out &out_img)
 {
-  using HL = HypLayout<D>;
-  constexpr int NV = HL::NV, LPC = HL::LPC;
+  using QL = QuadLayout<D>;
+  constexpr int LPC = QL::LPC;
   const LevelDesc &L = J.lv[level];
   const int w = L.w, h = L.h, hw = (w + 1) / 2;
   const int lane = threadIdx.x & 31, gl = lane & (LPC - 1);
+  const bool lane_on = QL::ACT == LPC || gl < QL::ACT;
   const int item = item0 + lane / LPC;
   int x = 0, y = 0;
   bool act = item < hw * h, skipped = false;
@@ -379,31 +411,29 @@ __device__ __forceinline__ void sweep_warp(const JobDesc &J, int level, int pari
     skipped = x < w && bp_skipped(J, level, x, y, kp.qt_max);
     act = x < w && !skipped;
   }
-  if (inherit && skipped)
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (inherit && skipped && lane_on)
   {
     // message inheritance of a cell the quadtree test skips at this level:
     // its messages keep the parent's (zeros at the coarsest level), as the
     // reference's copied-down images hold them (bpextract.cu:87-90,374-395);
     // half-sweeps 0 and 1 write them for their colour before any later
     // half-sweep reads them
-    const size_t c = (size_t)y * w + x;
+    const size_t c = ((size_t)y * w + x) * D + 4 * gl;
     const bool top = level + 1 >= J.nlev;
     const LevelDesc &C = J.lv[top ? level : level + 1];
-    const size_t pc = ((size_t)(y >> 1) * C.w + (x >> 1)) * D;
+    const size_t pc = ((size_t)(y >> 1) * C.w + (x >> 1)) * D + 4 * gl;
 #pragma unroll
     for (int m = 0; m < 4; ++m)
-#pragma unroll
-      for (int k = 0; k < NV; ++k)
-      {
-        const int d = gl + LPC * k;
-        out_img[m][c * D + d] = top ? 0.0f : msg_load<L2_ONLY>(C.msg[m] + pc + d);
-      }
+      *reinterpret_cast<float4 *>(out_img[m] + c) =
+          top ? zero : msg_load<L2_ONLY>(C.msg[m] + pc);
   }
   if (!__any_sync(0xffffffffu, act))
     return;
-  const bool has_u = act && y > 0, has_d = act && y < h - 1;
-  const bool has_l = act && x > 0, has_r = act && x < w - 1;
-  const size_t c = (size_t)y * w + x;
+  const bool on = act && lane_on;
+  const bool has_u = on && y > 0, has_d = on && y < h - 1;
+  const bool has_l = on && x > 0, has_r = on && x < w - 1;
+  const size_t c = ((size_t)y * w + x) * D + 4 * gl;
 
   // Incoming messages: the neighbours' own ones, or in the first half-sweep
   // of a level the ones their parents ended with (0 at the coarsest level),
@@ -411,43 +441,32 @@ __device__ __forceinline__ void sweep_warp(const JobDesc &J, int level, int pari
   const float *src_u = nullptr, *src_d = nullptr, *src_l = nullptr, *src_r = nullptr;
   if (!first)
   {
-    src_u = in[kDown] + (c - w) * D;
-    src_d = in[kUp] + (c + w) * D;
-    src_l = in[kRight] + (c - 1) * D;
-    src_r = in[kLeft] + (c + 1) * D;
+    src_u = in[kDown] + (c - (size_t)w * D);
+    src_d = in[kUp] + (c + (size_t)w * D);
+    src_l = in[kRight] + (c - D);
+    src_r = in[kLeft] + (c + D);
   }
   else if (level + 1 < J.nlev)
   {
     const LevelDesc &C = J.lv[level + 1];
-    auto parent = [&](int xn, int yn) { return ((size_t)(yn >> 1) * C.w + (xn >> 1)) * D; };
+    auto parent = [&](int xn, int yn) {
+      return ((size_t)(yn >> 1) * C.w + (xn >> 1)) * D + 4 * gl;
+    };
     src_u = C.msg[kDown] + parent(x, y - 1);
     src_d = C.msg[kUp] + parent(x, y + 1);
     src_l = C.msg[kRight] + parent(x - 1, y);
     src_r = C.msg[kLeft] + parent(x + 1, y);
   }
   const bool ld = src_u != nullptr;
-
-  float dat[NV], fu[NV], fd[NV], fl[NV], fr[NV];
-#pragma unroll
-  for (int k = 0; k < NV; ++k)
-  {
-    const int d = gl + LPC * k;
-    dat[k] = act ? L.data[c * D + d] : 0.0f;
-    fu[k] = (ld && has_u) ? msg_load<L2_ONLY>(src_u + d) : 0.0f;
-    fd[k] = (ld && has_d) ? msg_load<L2_ONLY>(src_d + d) : 0.0f;
-    fl[k] = (ld && has_l) ? msg_load<L2_ONLY>(src_l + d) : 0.0f;
-    fr[k] = (ld && has_r) ? msg_load<L2_ONLY>(src_r + d) : 0.0f;
-  }
-  cell_update<D, ARITH>(dat, fu, fd, fl, fr, has_u, has_d, has_l, has_r, kp, gl,
-                        [&](int dir, const float(&m)[NV], float mean) {
-                          if (act)
-                          {
-                            float *out = out_img[dir] + c * D;
-#pragma unroll
-                            for (int k = 0; k < NV; ++k)
-                              out[gl + LPC * k] = m[k] - mean;
-                          }
-                        });
+  const float4 dat = on ? *reinterpret_cast<const float4 *>(L.data + c) : zero;
+  const float4 fu = (ld && has_u) ? msg_load<L2_ONLY>(src_u) : zero;
+  const float4 fd = (ld && has_d) ? msg_load<L2_ONLY>(src_d) : zero;
+  const float4 fl = (ld && has_l) ? msg_load<L2_ONLY>(src_l) : zero;
+  const float4 fr = (ld && has_r) ? msg_load<L2_ONLY>(src_r) : zero;
+  cell_update<D, ARITH>(dat, fu, fd, fl, fr, kp, gl, [&](int dir, const float4 &v) {
+    if (on)
+      *reinterpret_cast<float4 *>(out_img[dir] + c) = v;
+  });
 }
 
 template <int D, int ARITH>
