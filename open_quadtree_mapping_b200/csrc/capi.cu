@@ -276,22 +276,19 @@ struct SoftBp
     const qm::Batch B = qm::stage::single(J);
     for (int l = 1; l < L; ++l)
       qm::launch_pyramid(B, cdiv_i((long)J.lv[l].w * J.lv[l].h * (D / 4), qm::kFlatThreads), l, s);
-    int lc = L;
-    while (lc > 0 && q.bp_iters[lc - 1] >= 2 &&
-           (long)J.lv[lc - 1].w * J.lv[lc - 1].h <= QM_DEFAULT_COARSE_CELLS)
-      --lc;
-    if (lc < L)
+    qm::CoarsePlan cp;
+    std::memset(&cp, 0, sizeof(cp));
+    cp.keep = 1;
+    long cells[qm::kMaxLevels] = {};
+    for (int l = 0; l < L; ++l)
     {
-      qm::CoarsePlan cp;
-      std::memset(&cp, 0, sizeof(cp));
-      cp.lo = lc;
-      cp.hi = L - 1;
-      cp.keep = 1;
-      for (int l = 0; l < L; ++l)
-      {
-        cp.iters[l] = q.bp_iters[l];
-        cp.hist[l] = hist_level(l);
-      }
+      cells[l] = (long)J.lv[l].w * J.lv[l].h;
+      cp.hist[l] = hist_level(l);
+    }
+    int lc = L;
+    if (qm::coarse_plan(cp, D, cells, L, q.bp_iters, QM_DEFAULT_COARSE_CELLS, 1, q.arith))
+    {
+      lc = cp.lo;
       qm::launch_bp_coarse(B, 0, 1, D, cp, kp, q.arith, s);
     }
     for (int l = lc - 1; l >= 0; --l)

@@ -87,7 +87,8 @@ struct StageTable
   std::vector<int> uniform;        // per stage: blocks per job when all agree, else 0
   std::vector<int> dvals;          // hypothesis counts present
   std::vector<size_t> level_bytes; // per job and BP level: data + messages
-  std::vector<long> level_cells;   // per BP level: largest cell count over the jobs
+  std::vector<int> job_d;          // per job: hypothesis count
+  std::vector<long> level_cells;   // per job and BP level: cells
   int max_w = 0, max_h = 0;        // longest lines of the row / column solves
   Tune tune;                       // launch shapes the blocks were counted for
 
@@ -112,6 +113,7 @@ struct StageTable
     }
     std::set<int> u(ds.begin(), ds.end());
     dvals.assign(u.begin(), u.end());
+    job_d = ds;
   }
 };
 
@@ -192,25 +194,30 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
       [&](const Batch &b, int g) { launch_cost(b, g, ar, max_d, s, T.tune.cost_blocks); });
   for (int l = 1; l < L; ++l)
     all(kPyramid, st.pyr(l), [&](const Batch &b, int g) { launch_pyramid(b, g, l, s); });
-  // BP, coarse to fine.  The top levels lc..L-1 whose cells are few (and
-  // which have two or more half-sweeps) run as one cluster launch per
-  // hypothesis count; below them each level runs job range by job range
-  // (message inheritance, half-sweeps, and at level 0 the extraction)
-  int lc = L;
-  if (coarse_cells > 0 && (int)T.level_cells.size() == L)
-    while (lc > 0 && p.bp_iters[lc - 1] >= 2 && T.level_cells[lc - 1] <= coarse_cells &&
-           in(st.sweep(lc - 1)))
-      --lc;
-  if (lc < L && jb > ja)
+  // BP, coarse to fine.  Per hypothesis count the top levels lc[..]..L-1 whose
+  // cells are few (and which have two or more half-sweeps) run as one cluster
+  // launch; below them each level runs job range by job range (message
+  // inheritance, half-sweeps, and at level 0 the extraction)
+  std::vector<int> lc(T.dvals.size(), L);
+  for (size_t di = 0; coarse_cells > 0 && di < T.dvals.size(); ++di)
   {
+    const int d = T.dvals[di];
+    long cells[kMaxLevels] = {};
+    int jobs = 0;
+    for (int j = ja; j < jb; ++j)
+      if (T.job_d[j] == d)
+      {
+        ++jobs;
+        for (int l = 0; l < L; ++l)
+          cells[l] = std::max(cells[l], T.level_cells[(size_t)j * L + l]);
+      }
     CoarsePlan cp;
     std::memset(&cp, 0, sizeof(cp));
-    cp.lo = lc;
-    cp.hi = L - 1;
-    for (int l = 0; l < L; ++l)
-      cp.iters[l] = p.bp_iters[l];
-    for (int d : T.dvals)
-      launch(kSweep, [&] { launch_bp_coarse(B, ja, jb - ja, d, cp, kp, ar, s); });
+    if (jobs == 0 || !in(st.sweep(L - 1)) ||
+        !coarse_plan(cp, d, cells, L, p.bp_iters, coarse_cells, jobs, ar))
+      continue;
+    lc[di] = cp.lo;
+    launch(kSweep, [&] { launch_bp_coarse(B, ja, jb - ja, d, cp, kp, ar, s); });
   }
   for (int l = L - 1; l >= 0; --l)
   {
@@ -222,9 +229,7 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
       // with two or more half-sweeps the first two write the inherited
       // messages themselves (no separate pass)
       const bool fold = p.bp_iters[l] >= 2;
-      if (l >= lc)
-        ; // swept by the coarse launch
-      else if (!fold && in(st.inherit(l)))
+      if (!fold && in(st.inherit(l)))
       {
         const Batch b = at(st.inherit(l), j0, j1, grid);
         if (grid > 0)
@@ -232,7 +237,7 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
             launch_msg_inherit(b, grid, l, p.bp_iters[l], p.qt_max_level, s);
           });
       }
-      if (l < lc && in(st.sweep(l)))
+      if (in(st.sweep(l)))
       {
         // consecutive half-sweeps walk the cells in opposite orders, so each
         // starts on the messages its predecessor wrote last (still in L2)
@@ -241,21 +246,25 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
           for (int it = 0; it < p.bp_iters[l]; ++it)
           {
             b.rev = it & 1;
-            for (int d : T.dvals)
-              launch(kSweep, [&] {
-                launch_bp_sweep(b, grid, d, l, it, kp, ar, s, T.tune.sweep_warps,
-                                fold && in(st.inherit(l)) ? 1 : 0);
-              });
+            for (size_t di = 0; di < T.dvals.size(); ++di)
+              if (l < lc[di])
+                launch(kSweep, [&] {
+                  launch_bp_sweep(b, grid, T.dvals[di], l, it, kp, ar, s, T.tune.sweep_warps,
+                                  fold && in(st.inherit(l)) ? 1 : 0);
+                });
           }
       }
       if (l == 0 && in(st.extract()))
       {
         // against the order of the level's last half-sweep (see above)
         Batch b = at(st.extract(), j0, j1, grid);
-        b.rev = (l < lc && p.bp_iters[0] > 0) ? 1 - ((p.bp_iters[0] - 1) & 1) : 0;
         if (grid > 0)
-          for (int d : T.dvals)
-            launch(kExtract, [&] { launch_extract(b, grid, d, ar, s, T.tune.extract_warps); });
+          for (size_t di = 0; di < T.dvals.size(); ++di)
+          {
+            b.rev = (lc[di] > 0 && p.bp_iters[0] > 0) ? 1 - ((p.bp_iters[0] - 1) & 1) : 0;
+            launch(kExtract,
+                   [&] { launch_extract(b, grid, T.dvals[di], ar, s, T.tune.extract_warps); });
+          }
       }
     }
   }
@@ -702,9 +711,8 @@ std::unique_ptr<TableBuf> Engine::build_table(const std::vector<int> &active, co
     for (int l = 0; l < L; ++l)
       T.level_bytes.push_back((size_t)5 * layouts_[j].lw[l] * layouts_[j].lh[l] * shapes_[j].D *
                               sizeof(float));
-    T.level_cells.resize(L, 0);
     for (int l = 0; l < L; ++l)
-      T.level_cells[l] = std::max(T.level_cells[l], (long)layouts_[j].lw[l] * layouts_[j].lh[l]);
+      T.level_cells.push_back((long)layouts_[j].lw[l] * layouts_[j].lh[l]);
   }
   T.add_jobs(per_job, ds);
   const int ns = (int)T.uniform.size();

@@ -21,6 +21,7 @@
 //
 // Bytes per updated cell and half-sweep: 9*D*4 (data + 4 messages read, 4
 // messages written).
+#include <atomic>
 #include <cfloat>
 #include <type_traits>
 
@@ -204,18 +205,9 @@ __global__ void __launch_bounds__(kFlatThreads)
 // bp kernel (bpextract.cu:200-312), one lane group per cell of the active
 // colour.  Groups whose cell is skipped or out of range still take part in
 // the warp's shuffles (full masks) with zero inputs and store nothing.
-//
-// msg_load: messages another block of the same launch may have written since
-// the launch began are read through L2 (ld.global.cg) by the coarse-level
-// kernel below, whose blocks hand messages to each other across cluster
-// barriers; the one-launch-per-half-sweep kernel reads them normally.
-template <bool L2_ONLY>
 __device__ __forceinline__ float4 msg_load(const float *p)
 {
-  if constexpr (L2_ONLY)
-    return __ldcg(reinterpret_cast<const float4 *>(p));
-  else
-    return *reinterpret_cast<const float4 *>(p);
+  return *reinterpret_cast<const float4 *>(p);
 }
 
 // ---- layout of the half-sweeps: lane g of a cell's group holds the four
@@ -390,7 +382,7 @@ __device__ __forceinline__ void cell_update(const float4 &dat, const float4 &fu,
 // neighbours' messages come from the images in[4], the cells' own go to
 // out[4], by direction (both the level's own ones, except where the soft BP
 // keeps the states between half-sweeps).
-template <int D, int ARITH, bool L2_ONLY, class In, class Out>
+template <int D, int ARITH, class In, class Out>
 __device__ __forceinline__ void sweep_warp(const JobDesc &J, int level, int parity, int first,
                                            int inherit, const KParams &kp, int item0, const In &in,
                                            const Out &out_img)
@@ -426,7 +418,7 @@ __device__ __forceinline__ void sweep_warp(const JobDesc &J, int level, int pari
 #pragma unroll
     for (int m = 0; m < 4; ++m)
       *reinterpret_cast<float4 *>(out_img[m] + c) =
-          top ? zero : msg_load<L2_ONLY>(C.msg[m] + pc);
+          top ? zero : msg_load(C.msg[m] + pc);
   }
   if (!__any_sync(0xffffffffu, act))
     return;
@@ -459,10 +451,10 @@ __device__ __forceinline__ void sweep_warp(const JobDesc &J, int level, int pari
   }
   const bool ld = src_u != nullptr;
   const float4 dat = on ? *reinterpret_cast<const float4 *>(L.data + c) : zero;
-  const float4 fu = (ld && has_u) ? msg_load<L2_ONLY>(src_u) : zero;
-  const float4 fd = (ld && has_d) ? msg_load<L2_ONLY>(src_d) : zero;
-  const float4 fl = (ld && has_l) ? msg_load<L2_ONLY>(src_l) : zero;
-  const float4 fr = (ld && has_r) ? msg_load<L2_ONLY>(src_r) : zero;
+  const float4 fu = (ld && has_u) ? msg_load(src_u) : zero;
+  const float4 fd = (ld && has_d) ? msg_load(src_d) : zero;
+  const float4 fl = (ld && has_l) ? msg_load(src_l) : zero;
+  const float4 fr = (ld && has_r) ? msg_load(src_r) : zero;
   cell_update<D, ARITH>(dat, fu, fd, fl, fr, kp, gl, [&](int dir, const float4 &v) {
     if (on)
       *reinterpret_cast<float4 *>(out_img[dir] + c) = v;
@@ -484,7 +476,7 @@ __global__ void __launch_bounds__(kMaxCellWarps * 32, 4)
   const int item0 = (lb * (int)(blockDim.x >> 5) + (threadIdx.x >> 5)) * G;
   if (item0 >= hw * L.h)
     return; // the whole warp
-  sweep_warp<D, ARITH, false>(J, level, parity, first, inherit, kp, item0, L.msg, L.msg);
+  sweep_warp<D, ARITH>(J, level, parity, first, inherit, kp, item0, L.msg, L.msg);
 }
 
 // Half-sweep `parity` from the message images io.in into io.out (the soft BP,
@@ -500,61 +492,271 @@ __global__ void __launch_bounds__(kMaxCellWarps * 32, 4)
   const int item0 = ((int)blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5)) * G;
   if (item0 >= (L.w + 1) / 2 * L.h)
     return; // the whole warp
-  sweep_warp<D, ARITH, false>(B.one, level, parity, first, 1, kp, item0, io.in, io.out);
+  sweep_warp<D, ARITH>(B.one, level, parity, first, 1, kp, item0, io.in, io.out);
 }
 
-// Every half-sweep of the coarse levels lo..hi (coarse to fine) in one
-// launch: a cluster of kCoarseCtas blocks per job walks the levels, each
-// half-sweep spread over the cluster's warps, with a cluster barrier (a
-// hardware barrier: release / acquire at cluster scope, no spinning) between
-// half-sweeps.  A coarse level's costs and messages (about 2.3 MB per
-// 752x480 job at levels 2 and 3 together) stay in L2 across its sweeps, and
-// its 10 half-sweeps no longer pay a launch and a grid drain each.  The
-// arithmetic is the per-half-sweep kernel's (the same device function), so
-// the messages are bit-identical; messages are read through L2 because other
-// blocks of the cluster wrote them.  Every block of a cluster takes the same
-// barriers: the trip counts depend only on the job and the plan.
+// Every half-sweep of the top levels lo..hi (coarse to fine) in one launch: a
+// cluster of plan.ctas blocks per job keeps a level in its shared memory.
 //
-// HIST: the half-sweeps read and write the plan's states (message_state), as
-// the adjoint of the soft BP needs them.
+// Bound: the latency of a half-sweep (a level has a few hundred to a few
+// thousand cells).  A launch per half-sweep costs 4 to 5 us, and so did
+// half-sweeps of one cluster launch that handed the messages on through L2;
+// here a half-sweep is shared-memory reads, the update and one hardware cluster
+// barrier (release / acquire, nothing spins).
+//
+// Layout: block r owns the cells [r per, (r + 1) per) of the level in row-major
+// order, with their edges to the right and to the lower neighbour.  An edge
+// holds ONE message, the one that will be read next: a half-sweep's cells all
+// have one colour, each reads its four edges and overwrites them with what it
+// sends, which the other colour reads in the next half-sweep.  That is 2 D
+// values per cell instead of 4 D, so 16 blocks hold about 7000 cells of 64
+// hypotheses; the data term stays in shared memory where it fits, in L2 where
+// not.  A cell's right and lower edge are its block's; its upper and left one
+// may be another block's (distributed shared memory).  A cell that the
+// quadtree test skips sends its inherited message all along: its edges hold
+// that one and are never overwritten.  Only the two last half-sweeps write the
+// level's message images (with HIST every one writes its kept state).
+// The update is the per-half-sweep kernel's device function, so the messages
+// are bit-identical.  Every block of a cluster takes the same barriers: the
+// trip counts depend only on the job and the plan.
+// Measured (the launch, one stream, messages through L2 with 8 blocks of 512
+// threads -> this one): 160x128 (34 half-sweeps) 113 -> 69 us, 752x480 (levels
+// 2 and 3) 99 -> 49, 1280x720 198 -> 79, 640x480 x 48 92 -> 47; clusters of 8
+// and 4 blocks: 752x480 76 and 105 us.
+struct CoarseCell
+{
+  unsigned short local, flags; // index in the block; CoarseFlag bits
+  unsigned short up_local, up_rank; // owner of the edge to the upper neighbour
+};
+enum CoarseFlag
+{
+  kHas = 1,    // << kUp .. kRight: the neighbour exists
+  kOpen = 16,  // << kUp .. kRight: it exists and is not skipped
+  kSkip = 256, // the cell itself is skipped
+};
+
+__device__ __forceinline__ unsigned cluster_rank()
+{
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier()
+{
+  asm volatile("barrier.cluster.arrive.release.aligned;\n"
+               "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// the address of p (this block's shared memory) in the block `rank`
+__device__ __forceinline__ unsigned cluster_addr(const float *p, unsigned rank)
+{
+  unsigned a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;"
+      : "=r"(a)
+      : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float4 cluster_load(unsigned a)
+{
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(a)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_store(unsigned a, const float4 &v)
+{
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y),
+               "f"(v.z), "f"(v.w)
+               : "memory");
+}
+
+// shared memory of a block with `per` cells, in floats: edges, data term, and
+// the cell lists of the two colours, the flags and the list lengths behind it
+template <int D>
+__host__ __device__ constexpr size_t coarse_smem(int per, bool with_data)
+{
+  return (size_t)per * (2 + (with_data ? 1 : 0)) * D * sizeof(float) +
+         (size_t)per * (2 * sizeof(CoarseCell) + sizeof(unsigned short)) + 32;
+}
+
 template <int D, int ARITH, bool HIST>
-__global__ void __cluster_dims__(kCoarseCtas, 1, 1) __launch_bounds__(kCoarseThreads, 2)
+__global__ void __launch_bounds__(kCoarseMaxThreads, 1)
     k_bp_coarse(const __grid_constant__ Batch B, int j0, const __grid_constant__ CoarsePlan plan,
                 KParams kp)
 {
-  constexpr int G = HypLayout<D>::G;
-  const int job = j0 + (int)blockIdx.x / kCoarseCtas;
+  using QL = QuadLayout<D>;
+  constexpr int LPC = QL::LPC, G = 32 / LPC;
+  const int threads = blockDim.x, groups = threads / LPC;
+  extern __shared__ __align__(16) float s_coarse[];
+  const int ctas = plan.ctas;
+  const int job = j0 + (int)blockIdx.x / ctas;
   const JobDesc &J = B.jobs ? B.jobs[job] : B.one;
   if (J.D != D)
     return; // the whole cluster
-  const int warps = kCoarseThreads / 32;
-  const int gw = (int)(blockIdx.x % kCoarseCtas) * warps + (int)(threadIdx.x >> 5);
-  const int stride = kCoarseCtas * warps * G;
+  const int rank = (int)cluster_rank();
+  const int tid = threadIdx.x, lane = tid & 31, gl = lane & (LPC - 1), group = tid / LPC;
+  const bool lane_on = QL::ACT == LPC || gl < QL::ACT;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float *edges = s_coarse;
+  float *data = s_coarse + (size_t)plan.per * 2 * D;
+  CoarseCell *lists =
+      reinterpret_cast<CoarseCell *>(data + (plan.data_smem ? (size_t)plan.per * D : 0));
+  unsigned short *flags = reinterpret_cast<unsigned short *>(lists + 2 * plan.per);
+  __shared__ int s_len[2];
   for (int level = plan.hi; level >= plan.lo; --level)
   {
     const LevelDesc &L = J.lv[level];
-    const int n = (L.w + 1) / 2 * L.h;
+    const int w = L.w, h = L.h, n = w * h;
+    const int per = (n + ctas - 1) / ctas;
+    const int c0 = rank * per, cnt = max(0, min(per, n - c0));
     const int iters = plan.iters[level];
+    const bool top = level + 1 >= J.nlev;
+    const LevelDesc &P = J.lv[top ? level : level + 1];
+    // ---- flags of the block's cells
+    for (int i = tid; i < cnt; i += threads)
+    {
+      const int c = c0 + i, y = c / w, x = c - y * w;
+      auto skip = [&](int xn, int yn) { return bp_skipped(J, level, xn, yn, kp.qt_max); };
+      unsigned f = skip(x, y) ? kSkip : 0;
+      if (y > 0)
+        f |= (skip(x, y - 1) ? kHas : kHas | kOpen) << kUp;
+      if (y < h - 1)
+        f |= (skip(x, y + 1) ? kHas : kHas | kOpen) << kDown;
+      if (x > 0)
+        f |= (skip(x - 1, y) ? kHas : kHas | kOpen) << kLeft;
+      if (x < w - 1)
+        f |= (skip(x + 1, y) ? kHas : kHas | kOpen) << kRight;
+      flags[i] = (unsigned short)f;
+    }
+    __syncthreads();
+    // ---- the cells that are swept, by colour (warps 0 and 1, in order)
+    if (tid < 64)
+    {
+      const int colour = tid >> 5;
+      int len = 0;
+      for (int i0 = 0; i0 < cnt; i0 += 32)
+      {
+        const int i = i0 + lane, c = c0 + i, y = c / w, x = c - y * w;
+        const bool in = i < cnt && ((x + y) & 1) == colour && !(flags[i] & kSkip);
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in)
+        {
+          const int up = max(c - w, 0), r = up / per;
+          lists[colour * plan.per + len + __popc(m & ((1u << lane) - 1u))] =
+              CoarseCell{(unsigned short)i, flags[i], (unsigned short)(up - r * per),
+                         (unsigned short)r};
+        }
+        len += __popc(m);
+      }
+      if (lane == 0)
+        s_len[colour] = len;
+    }
+    // ---- starting messages: an edge gets the message from its odd cell (read
+    // by half-sweep 0), or from its even cell where that one is skipped; the
+    // parents' final messages, 0 at the coarsest level (what the reference's
+    // copied-down messages hold, bpextract.cu:87-90,374-395)
+    if (lane_on)
+    {
+      auto parent = [&](int m, int x, int y) {
+        return top ? zero
+                   : __ldcg(reinterpret_cast<const float4 *>(
+                         P.msg[m] + ((size_t)(y >> 1) * P.w + (x >> 1)) * D + 4 * gl));
+      };
+      for (int i = group; i < cnt; i += groups)
+      {
+        const int c = c0 + i, y = c / w, x = c - y * w;
+        const unsigned f = flags[i];
+        const bool even = ((x + y) & 1) == 0;
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+        {
+          const int to = e == 0 ? kRight : kDown, back = e == 0 ? kLeft : kUp;
+          if (!(f & (kHas << to)))
+            continue;
+          const bool even_skipped = even ? (f & kSkip) != 0 : !(f & (kOpen << to));
+          const bool mine = even == even_skipped; // this cell's message, or the neighbour's
+          const float4 v = mine ? parent(to, x, y) : parent(back, x + (e == 0), y + (e == 1));
+          *reinterpret_cast<float4 *>(edges + ((size_t)i * 2 + e) * D + 4 * gl) = v;
+        }
+        if (plan.data_smem)
+          *reinterpret_cast<float4 *>(data + (size_t)i * D + 4 * gl) =
+              *reinterpret_cast<const float4 *>(L.data + (size_t)c * D + 4 * gl);
+        if (f & kSkip)
+        {
+#pragma unroll
+          for (int m = 0; m < 4; ++m)
+          {
+            const float4 v = parent(m, x, y);
+            const size_t o = (size_t)c * D + 4 * gl;
+            *reinterpret_cast<float4 *>(L.msg[m] + o) = v;
+            if constexpr (HIST)
+              for (int it = iters - 3; it >= 0; it -= 2)
+                *reinterpret_cast<float4 *>(plan.hist[level].at(it, iters, m, L.msg[m]) + o) = v;
+          }
+        }
+      }
+    }
+    cluster_barrier();
+    // ---- half-sweeps
     for (int it = 0; it < iters; ++it)
     {
-      if constexpr (HIST)
-      {
-        float *in[4], *out[4];
+      const CoarseCell *list = lists + (it & 1) * plan.per;
+      const int len = s_len[it & 1];
+      const bool out_on = HIST || it >= iters - 2;
+      float *out[4];
 #pragma unroll
-        for (int m = 0; m < 4; ++m)
+      for (int m = 0; m < 4; ++m)
+        out[m] = HIST ? plan.hist[level].at(it, iters, m, L.msg[m]) : L.msg[m];
+      for (int k0 = (tid >> 5) * G; k0 < len; k0 += threads / LPC)
+      {
+        const int k = k0 + lane / LPC;
+        const bool on = k < len && lane_on;
+        const CoarseCell q = list[min(k, len - 1)];
+        const unsigned f = q.flags;
+        const int i = q.local;
+        float *own = edges + (size_t)i * 2 * D + 4 * gl;
+        // the edges to the left (the previous cell's first) and up
+        const bool far_l = i == 0, far_u = (int)q.up_rank != rank;
+        float *left = edges + (size_t)(far_l ? per - 1 : i - 1) * 2 * D + 4 * gl;
+        float *up = edges + ((size_t)q.up_local * 2 + 1) * D + 4 * gl;
+        const unsigned left_a = far_l ? cluster_addr(left, max(rank - 1, 0)) : 0u;
+        const unsigned up_a = far_u ? cluster_addr(up, q.up_rank) : 0u;
+        float4 fu = zero, fd = zero, fl = zero, fr = zero, dat = zero;
+        if (on)
         {
-          in[m] = plan.hist[level].at(it - 1, iters, m, L.msg[m]);
-          out[m] = plan.hist[level].at(it, iters, m, L.msg[m]);
+          dat = plan.data_smem
+                    ? *reinterpret_cast<const float4 *>(data + (size_t)i * D + 4 * gl)
+                    : __ldg(reinterpret_cast<const float4 *>(L.data + (size_t)(c0 + i) * D +
+                                                             4 * gl));
+          if (f & (kHas << kUp))
+            fu = far_u ? cluster_load(up_a) : *reinterpret_cast<const float4 *>(up);
+          if (f & (kHas << kLeft))
+            fl = far_l ? cluster_load(left_a) : *reinterpret_cast<const float4 *>(left);
+          if (f & (kHas << kRight))
+            fr = *reinterpret_cast<const float4 *>(own);
+          if (f & (kHas << kDown))
+            fd = *reinterpret_cast<const float4 *>(own + D);
         }
-        for (int item0 = gw * G; item0 < n; item0 += stride)
-          sweep_warp<D, ARITH, true>(J, level, it & 1, it == 0 ? 1 : 0, 1, kp, item0, in, out);
+        cell_update<D, ARITH>(dat, fu, fd, fl, fr, kp, gl, [&](int dir, const float4 &v) {
+          if (!on)
+            return;
+          if (f & (kOpen << dir))
+          {
+            if (dir == kRight)
+              *reinterpret_cast<float4 *>(own) = v;
+            else if (dir == kDown)
+              *reinterpret_cast<float4 *>(own + D) = v;
+            else if (dir == kLeft ? far_l : far_u)
+              cluster_store(dir == kLeft ? left_a : up_a, v);
+            else
+              *reinterpret_cast<float4 *>(dir == kLeft ? left : up) = v;
+          }
+          if (out_on)
+            *reinterpret_cast<float4 *>(out[dir] + (size_t)(c0 + i) * D + 4 * gl) = v;
+        });
       }
-      else
-        for (int item0 = gw * G; item0 < n; item0 += stride)
-          sweep_warp<D, ARITH, true>(J, level, it & 1, it == 0 ? 1 : 0, it < 2 ? 1 : 0, kp, item0,
-                                     L.msg, L.msg);
-      asm volatile("barrier.cluster.arrive.release.aligned;\n"
-                   "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+      cluster_barrier();
     }
   }
 }
@@ -678,15 +880,94 @@ void sweep_d(const Batch &B, int blocks, int level, int parity, int first, int i
         <<<blocks, warps * 32, 0, s>>>(B, level, parity, first, inherit, kp);
 }
 
-template <int D, bool HIST>
+// Opt-ins of one k_bp_coarse instance on the current device (large shared
+// memory, clusters of 16); true when the device can hold such a cluster.
+template <int D, int ARITH, bool HIST>
+bool coarse_prepare(int ctas)
+{
+  static std::atomic<unsigned long long> done{0}, wide{0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess)
+    return false;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (!(done.load(std::memory_order_acquire) & bit))
+  {
+    const auto k = k_bp_coarse<D, ARITH, HIST>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem - 64);
+    cudaLaunchConfig_t c = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kCoarseMaxCtas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    c.gridDim = dim3(kCoarseMaxCtas);
+    c.blockDim = dim3(kCoarseMaxThreads);
+    c.dynamicSmemBytes = kMaxBlockSmem - 64;
+    c.attrs = at;
+    c.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+            cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, k, &c) == cudaSuccess && clusters > 0)
+      wide.fetch_or(bit, std::memory_order_acq_rel);
+    cudaGetLastError(); // a device without such clusters is no error
+    done.fetch_or(bit, std::memory_order_acq_rel);
+  }
+  return ctas <= 8 || (wide.load(std::memory_order_acquire) & bit);
+}
+
+template <int D, int ARITH, bool HIST>
+void coarse_k(const Batch &B, int j0, int jobs, const CoarsePlan &plan, KParams kp, cudaStream_t s)
+{
+  coarse_prepare<D, ARITH, HIST>(plan.ctas);
+  cudaLaunchConfig_t c = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = plan.ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  c.gridDim = dim3(jobs * plan.ctas);
+  c.blockDim = dim3(plan.threads);
+  c.dynamicSmemBytes = coarse_smem<D>(plan.per, plan.data_smem != 0);
+  c.stream = s;
+  c.attrs = at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, k_bp_coarse<D, ARITH, HIST>, B, j0, plan, kp);
+}
+
+template <int D>
 void coarse_d(const Batch &B, int j0, int jobs, const CoarsePlan &plan, KParams kp, int arith,
               cudaStream_t s)
 {
-  const int g = jobs * kCoarseCtas;
+  constexpr int R = QM_ARITH_REFERENCE, I = QM_ARITH_IEEE;
   if (arith == QM_ARITH_IEEE)
-    k_bp_coarse<D, QM_ARITH_IEEE, HIST><<<g, kCoarseThreads, 0, s>>>(B, j0, plan, kp);
+    plan.keep ? coarse_k<D, I, true>(B, j0, jobs, plan, kp, s)
+              : coarse_k<D, I, false>(B, j0, jobs, plan, kp, s);
   else
-    k_bp_coarse<D, QM_ARITH_REFERENCE, HIST><<<g, kCoarseThreads, 0, s>>>(B, j0, plan, kp);
+    plan.keep ? coarse_k<D, R, true>(B, j0, jobs, plan, kp, s)
+              : coarse_k<D, R, false>(B, j0, jobs, plan, kp, s);
+}
+
+template <int D>
+bool coarse_fit_d(CoarsePlan &plan, long cells, int ctas, bool shared_sm, int arith)
+{
+  constexpr int R = QM_ARITH_REFERENCE, I = QM_ARITH_IEEE;
+  const long per = (cells + ctas - 1) / ctas;
+  constexpr size_t room = kMaxBlockSmem - 64; // 64: s_len
+  if (per > 4096 || coarse_smem<D>((int)per, false) > room)
+    return false;
+  const bool can = arith == QM_ARITH_IEEE
+                       ? (plan.keep ? coarse_prepare<D, I, true>(ctas) : coarse_prepare<D, I, false>(ctas))
+                       : (plan.keep ? coarse_prepare<D, R, true>(ctas) : coarse_prepare<D, R, false>(ctas));
+  if (!can)
+    return false;
+  plan.ctas = ctas;
+  plan.per = (int)per;
+  // two blocks per SM: half the threads each, and half the shared memory if
+  // that is possible without the data term
+  const size_t half = kMaxBlockSmem / 2 - 2048;
+  const bool split = shared_sm && coarse_smem<D>((int)per, false) <= half;
+  plan.threads = split ? 512 : kCoarseMaxThreads;
+  plan.data_smem = coarse_smem<D>((int)per, true) <= (split ? half : room) ? 1 : 0;
+  return true;
 }
 
 template <int D>
@@ -795,15 +1076,38 @@ void launch_bp_sweep_io(const Batch &B, int d, int level, int it, const SweepIO 
     });
 }
 
+bool coarse_plan(CoarsePlan &plan, int d, const long *cells, int levels, const int *iters,
+                 long max_cells, int jobs, int arith)
+{
+  plan.lo = levels;
+  plan.hi = levels - 1;
+  for (int l = 0; l < levels; ++l)
+    plan.iters[l] = iters[l];
+  // Few jobs: the widest cluster for each (a half-sweep's latency counts).
+  // Above kCoarseWideJobs clusters of 16 no longer run all at once (148 SMs);
+  // then 8 blocks of 512 threads per job, two on an SM, if the level fits them
+  // (32 x 752x480, all half-sweeps: 0.965 ms; one 1024-thread block per SM
+  // 1.055, the former launch 0.985).
+  const int first = jobs <= kCoarseWideJobs ? kCoarseMaxCtas : 8;
+  for (int l = levels - 1; l >= 0 && iters[l] >= 2 && cells[l] <= max_cells; --l)
+  {
+    bool ok = false;
+    by_d(d, [&](auto dc) {
+      constexpr int D = decltype(dc)::value;
+      ok = coarse_fit_d<D>(plan, cells[l], first, first == 8, arith) ||
+           coarse_fit_d<D>(plan, cells[l], first == 8 ? kCoarseMaxCtas : 8, first == 8, arith);
+    });
+    if (!ok)
+      break;
+    plan.lo = l;
+  }
+  return plan.lo < levels;
+}
+
 void launch_bp_coarse(const Batch &B, int j0, int jobs, int d, const CoarsePlan &plan,
                       KParams kp, int arith, cudaStream_t s)
 {
-  by_d(d, [&](auto dc) {
-    if (plan.keep)
-      coarse_d<decltype(dc)::value, true>(B, j0, jobs, plan, kp, arith, s);
-    else
-      coarse_d<decltype(dc)::value, false>(B, j0, jobs, plan, kp, arith, s);
-  });
+  by_d(d, [&](auto dc) { coarse_d<decltype(dc)::value>(B, j0, jobs, plan, kp, arith, s); });
 }
 
 void launch_extract(const Batch &B, int blocks, int d, int arith, cudaStream_t s, int warps)

@@ -96,19 +96,28 @@ struct SweepIO
 // messages) into io.out, skipped cells included
 void launch_bp_sweep_io(const Batch &B, int d, int level, int it, const SweepIO &io, KParams kp,
                         int arith, cudaStream_t s);
-// Coarse BP levels in one launch (k_bp_coarse): levels hi down to lo, every
-// one with at least two half-sweeps (their first two write the inherited
-// messages), one cluster of kCoarseCtas blocks of kCoarseThreads threads per
-// job, jobs j0 .. j0 + jobs - 1 of the batch (B.jobs null: the inline job).
-constexpr int kCoarseCtas = 8;
-constexpr int kCoarseThreads = 512;
+// Top BP levels in one launch (k_bp_coarse): levels hi down to lo, every one
+// with at least two half-sweeps, a cluster of `ctas` blocks per job keeping a
+// level in shared memory, `per` cells per block.
+constexpr int kCoarseMaxThreads = 1024;
+constexpr int kCoarseMaxCtas = 16; // above the portable 8: asked of the device
+constexpr int kCoarseWideJobs = 8; // jobs that get clusters of 16 blocks
 struct CoarsePlan
 {
   int lo, hi;
   int iters[kMaxLevels];
-  int keep; // 1: the half-sweeps keep their states in hist
+  int ctas, per, threads;
+  int data_smem; // 1: the data term in shared memory too
+  int keep;      // 1: the half-sweeps keep their states in hist
   HistLevel hist[kMaxLevels];
 };
+// Sizes the plan for `jobs` jobs of d hypotheses: the top levels with at most
+// max_cells cells in every job (cells[l]: the most), two half-sweeps or more,
+// and room in a cluster's shared memory.  False: no such level.  plan.keep is
+// read, the rest (but hist) written.
+bool coarse_plan(CoarsePlan &plan, int d, const long *cells, int levels, const int *iters,
+                 long max_cells, int jobs, int arith);
+// jobs j0 .. j0 + jobs - 1 of the batch (B.jobs null: the inline job)
 void launch_bp_coarse(const Batch &B, int j0, int jobs, int d, const CoarsePlan &plan,
                       KParams kp, int arith, cudaStream_t s);
 void launch_extract(const Batch &B, int blocks, int d, int arith, cudaStream_t s,
