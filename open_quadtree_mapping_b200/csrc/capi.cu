@@ -1280,7 +1280,9 @@ int qm_semidense_step(const uint8_t *key, const uint8_t *inc, int width, int hei
         throw CudaError{QM_ERR_CUDA, "texture object creation failed"};
       }
     }
-    qm::launch_semidense(B, qm::sd_blocks(width, height), ref ? 0 : 1, s);
+    B.tile = qm::sd_tile((long)width * height);
+    qm::launch_semidense(B, qm::sd_blocks(width, height), qm::sd_tiles(width, height, B.tile),
+                         ref ? 0 : 1, s);
     const cudaError_t e = cudaGetLastError();
     if (ref)
     {

@@ -46,6 +46,7 @@ namespace
 {
 
 constexpr int kSdThreads = 256;
+constexpr int kSdTile = 1024; // most pixels of one block of the stereo update
 constexpr unsigned long long kSdEmpty = ~0ull;
 
 // reference constants (stereo_parameter.cuh:1-41)
@@ -130,7 +131,7 @@ __device__ __forceinline__ int trunc_plus_half(float v) { return (int)((double)v
 
 // ---------------------------------------------------------------------------
 // The job of a block (block prefix over the streams of the step).
-__device__ __forceinline__ const SdJob &sd_job(const SdBatch &B, int &lb)
+__device__ __forceinline__ const SdJob &sd_job(const SdBatch &B, const int *prefix, int &lb)
 {
   const int block = (int)blockIdx.x;
   if (B.jobs == nullptr)
@@ -138,9 +139,13 @@ __device__ __forceinline__ const SdJob &sd_job(const SdBatch &B, int &lb)
     lb = block;
     return B.one;
   }
-  const int j = find_job(B.prefix, B.njobs, block);
-  lb = block - __ldg(B.prefix + j);
+  const int j = find_job(prefix, B.njobs, block);
+  lb = block - __ldg(prefix + j);
   return B.jobs[j];
+}
+__device__ __forceinline__ const SdJob &sd_job(const SdBatch &B, int &lb)
+{
+  return sd_job(B, B.prefix, lb);
 }
 
 // pixel of this thread, false when outside the image
@@ -277,6 +282,25 @@ __global__ void __launch_bounds__(kSdThreads) k_sd_init(const __grid_constant__ 
   store_seed(J, 0, o, s);
 }
 
+// The pose and camera of a job as values the optimiser knows nothing about.
+// A kernel that loops over pixels would otherwise compute products of them
+// once, outside the loop, where they no longer fuse with the addition they
+// belong to: reference arithmetic would round differently.
+struct View
+{
+  float T[12], fx, fy, cx, cy;
+  __device__ __forceinline__ explicit View(const SdJob &J) : fx(J.fx), fy(J.fy), cx(J.cx), cy(J.cy)
+  {
+#pragma unroll
+    for (int k = 0; k < 12; ++k)
+    {
+      T[k] = J.T[k];
+      asm volatile("" : "+f"(T[k]));
+    }
+    asm volatile("" : "+f"(fx), "+f"(fy), "+f"(cx), "+f"(cy));
+  }
+};
+
 // Sum of the products of two five-sample residual sets, left to right.
 template <bool I>
 __device__ __forceinline__ Fl<I> residual_overlap(const Fl<I> (&a)[5], const Fl<I> (&b)[5])
@@ -296,8 +320,9 @@ __device__ float search_point(const SdJob &J, int x, int y, float2 epi, Fl<I> gr
                               Fl<I> &result_idep, Fl<I> &result_var)
 {
   using F = Fl<I>;
-  const F fx(J.fx), fy(J.fy), cx(J.cx), cy(J.cy);
-  const float *T = J.T;
+  const View V(J);
+  const F fx(V.fx), fy(V.fy), cx(V.cx), cy(V.cy);
+  const float *T = V.T;
   // five keyframe samples along the epipolar direction, centred on (x, y)
   F key_patch[5];
 #pragma unroll
@@ -359,41 +384,33 @@ __device__ float search_point(const SdJob &J, int x, int y, float2 epi, Fl<I> gr
   F prev_score(1e9f), score(1e9f);
   // the sample of step s + 1 is fetched while step s is scored (sampling is
   // a pure function of its coordinates and clamps, so the fetch past the last
-  // step is harmless)
-  auto fetch = [&](int step) {
-    const F sx = far_u + F((float)step) * dir_u, sy = far_v + F((float)step) * dir_v;
+  // step is harmless); its position is the next step's
+  auto fetch = [&](F sx, F sy) {
     return sample<I>(J.inc_tex, J.inc_f, J.pitch, J.W, J.H,
                      (float)((double)sx.v + 2.0 * (double)dir_u.v + 0.5),
                      (float)((double)sy.v + 2.0 * (double)dir_v.v + 0.5));
   };
-  F next = fetch(0);
-  for (int step = 0; (float)step <= search_length.v && step <= kMaxSearch; step += 1)
-  {
+  // the step as a float (exact), counted up instead of converted
+  float at = 0.0f;
+  F sx = far_u + F(at) * dir_u, sy = far_v + F(at) * dir_v;
+  F next = fetch(sx, sy);
+  const float u_end = (float)(J.W - 1), v_end = (float)(J.H - 1);
+  // one step; res: the residuals of this parity.  False: the line left the image
+  auto take = [&](F(&res)[5]) {
     prev_score = score;
     score = F(0.0f);
-    const F sx = far_u + F((float)step) * dir_u, sy = far_v + F((float)step) * dir_v;
-    if (sx.v <= 1.0f || sx.v >= (float)(J.W - 1) || sy.v <= 1.0f || sy.v >= (float)(J.H - 1))
-      break;
+    if (sx.v <= 1.0f || sx.v >= u_end || sy.v <= 1.0f || sy.v >= v_end)
+      return false;
     line_patch[4] = next;
-    next = fetch(step + 1);
+    sx = far_u + F(at + 1.0f) * dir_u;
+    sy = far_v + F(at + 1.0f) * dir_v;
+    next = fetch(sx, sy);
     // squared residuals, newest sample first
-    if (step % 2 == 0)
-    {
 #pragma unroll
-      for (int j = 0; j < 5; ++j)
-      {
-        res_even[j] = line_patch[4 - j] - key_patch[4 - j];
-        score = score + res_even[j] * res_even[j];
-      }
-    }
-    else
+    for (int j = 0; j < 5; ++j)
     {
-#pragma unroll
-      for (int j = 0; j < 5; ++j)
-      {
-        res_odd[j] = line_patch[4 - j] - key_patch[4 - j];
-        score = score + res_odd[j] * res_odd[j];
-      }
+      res[j] = line_patch[4 - j] - key_patch[4 - j];
+      score = score + res[j] * res[j];
     }
     if (last_is_best)
     {
@@ -406,7 +423,7 @@ __device__ float search_point(const SdJob &J, int x, int y, float2 epi, Fl<I> gr
       second_best_score = best_score;
       second_best_step = best_step;
       best_score = score;
-      best_step = F((float)step);
+      best_step = F(at);
       score_before_best = prev_score;
       overlap_before = residual_overlap<I>(res_even, res_odd);
       overlap_after = F(-1.0f);
@@ -416,11 +433,19 @@ __device__ float search_point(const SdJob &J, int x, int y, float2 epi, Fl<I> gr
     else if (score < second_best_score)
     {
       second_best_score = score;
-      second_best_step = F((float)step);
+      second_best_step = F(at);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       line_patch[j] = line_patch[j + 1];
+    at += 1.0f;
+    return true;
+  };
+  const float last = search_length.v > (float)kMaxSearch ? (float)kMaxSearch : search_length.v;
+  while (at <= last)
+  {
+    if (!take(res_even) || !(at <= last) || !take(res_odd))
+      break;
   }
 
   if (best_score > F(4.0f * kMaxErrorStereo))
@@ -500,50 +525,109 @@ __device__ float search_point(const SdJob &J, int x, int y, float2 epi, Fl<I> gr
   return best_score.v;
 }
 
-// update_keyframe_kernel (lsd_semidense.cu:400-515): one stereo observation
-// per seed; reads and writes only its own seed.
-// 4 blocks per SM (at most 64 registers instead of 86 / 102, i.e. 2 blocks):
-// the search loop is latency-bound, and the extra resident warps outweigh
-// the spilled values (tracker per stream and frame at 752x480: 0.171 ms at
-// 2 blocks, 0.144 at 3, 0.127 at 4, 0.125 at 5)
+// The gates of update_keyframe_kernel (lsd_semidense.cu:400-440) before its
+// search: false where the pixel gets no observation this frame.
 template <bool I>
-__global__ void __launch_bounds__(kSdThreads, 4) k_sd_update(const __grid_constant__ SdBatch B)
+__device__ __forceinline__ bool observable(const SdJob &J, int x, int y, Fl<I> &gradient_max,
+                                           Fl<I> &gae, float2 &epi)
 {
   using F = Fl<I>;
-  int lb, x, y;
-  const SdJob &J = sd_job(B, lb);
-  if (J.mode < kSdUpdate || !sd_pixel(J, lb, x, y) || !sd_interior(J, x, y))
-    return;
+  if (!sd_interior(J, x, y))
+    return false;
   const float2 g = grad_at(J.key_f, J.pitch, x, y);
-  const F gradient_max = fsqrt(dot2<I>(g));
+  gradient_max = fsqrt(dot2<I>(g));
   if (gradient_max < F(kMinGrad))
-    return;
-  const size_t o = (size_t)y * J.W + x;
-  Seed s = load_seed(J, 0, o);
-  if (s.t.y < kMinBlacklist)
-    return;
-  const bool first_observe = !valid(s);
-  const float *T = J.T;
+    return false;
+  if (J.trk[J.cur][(size_t)y * J.W + x].y < kMinBlacklist)
+    return false;
+  const View V(J);
+  const float *T = V.T;
   // translation of the inverse of T (se3.cuh:91-107)
   const F itx = -F(T[0]) * F(T[3]) - F(T[4]) * F(T[7]) - F(T[8]) * F(T[11]);
   const F ity = -F(T[1]) * F(T[3]) - F(T[5]) * F(T[7]) - F(T[9]) * F(T[11]);
   const F itz = -F(T[2]) * F(T[3]) - F(T[6]) * F(T[7]) - F(T[10]) * F(T[11]);
-  F ex = -F(J.fx) * itx + itz * (F((float)x) - F(J.cx));
-  F ey = -F(J.fy) * ity + itz * (F((float)y) - F(J.cy));
+  F ex = -F(V.fx) * itx + itz * (F((float)x) - F(V.cx));
+  F ey = -F(V.fy) * ity + itz * (F((float)y) - F(V.cy));
   const F epi_length = fsqrt(ex * ex + ey * ey);
   if ((double)epi_length.v < 1.0)
-    return;
+    return false;
   ex = ex / epi_length;
   ey = ey / epi_length;
-  const F gae = F(fabsf((ex * F(g.x) + ey * F(g.y)).v));
+  gae = F(fabsf((ex * F(g.x) + ey * F(g.y)).v));
   if ((double)gae.v < 2.0)
-    return;
+    return false;
   if ((double)(gae / gradient_max).v < 0.3)
-    return;
+    return false;
+  epi = make_float2(ex.v, ey.v);
+  return true;
+}
 
+template <bool I>
+__device__ __forceinline__ void update_seed(const SdJob &J, int x, int y, Fl<I> gradient_max,
+                                            Fl<I> gae, float2 epi);
+
+// update_keyframe_kernel (lsd_semidense.cu:400-515): one stereo observation
+// per seed; reads and writes only its own seed.
+// Bound: the search loop (up to 101 samples per observed seed, each a texture
+// fetch and about 60 instructions).  A block first collects the pixels of its
+// tile that will be searched, so that the warps of the loop are full (on
+// textured frames about half of the pixels pass the gates, scattered, and
+// almost every warp of consecutive pixels had some).  Nine streams of 624x408
+// to 1264x816: the step 1.37 -> 0.84 ms without the neighbourhood passes.
+// 4 blocks per SM (at most 64 registers instead of 86 / 102, i.e. 2 blocks):
+// the search loop is latency-bound, and the extra resident warps outweigh
+// the spilled values (tracker per stream and frame at 752x480: 0.171 ms at
+// 2 blocks, 0.144 at 3, 0.127 at 4, 0.125 at 5).
+template <bool I>
+__global__ void __launch_bounds__(kSdThreads, 4) k_sd_update(const __grid_constant__ SdBatch B)
+{
+  using F = Fl<I>;
+  __shared__ unsigned short s_list[kSdTile];
+  __shared__ int s_count;
+  int lb;
+  const SdJob &J = sd_job(B, B.tile_prefix, lb);
+  if (J.mode < kSdUpdate)
+    return; // the whole block
+  const int W = J.W, n = W * J.H, tile = B.tile, base = lb * tile;
+  if (threadIdx.x == 0)
+    s_count = 0;
+  __syncthreads();
+  F gradient_max, gae;
+  float2 epi;
+  const int lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < tile; i += kSdThreads)
+  {
+    const int p = base + i, y = p / W, x = p - y * W;
+    const bool on = p < n && observable<I>(J, x, y, gradient_max, gae, epi);
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    int at = 0;
+    if (lane == 0 && m)
+      at = atomicAdd(&s_count, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (on)
+      s_list[at + __popc(m & ((1u << lane) - 1u))] = (unsigned short)i;
+  }
+  __syncthreads();
+  const int count = s_count;
+  for (int i = threadIdx.x; i < count; i += kSdThreads)
+  {
+    const int p = base + s_list[i], y = p / W, x = p - y * W;
+    observable<I>(J, x, y, gradient_max, gae, epi);
+    update_seed<I>(J, x, y, gradient_max, gae, epi);
+  }
+}
+
+template <bool I>
+__device__ __forceinline__ void update_seed(const SdJob &J, int x, int y, Fl<I> gradient_max,
+                                            Fl<I> gae, float2 epi)
+{
+  using F = Fl<I>;
+  const size_t o = (size_t)y * J.W + x;
+  Seed s = load_seed(J, 0, o);
+  const bool first_observe = !valid(s);
   F result_idep(0.0f), result_var(0.0f);
-  const float err = search_point<I>(J, x, y, make_float2(ex.v, ey.v), gradient_max, gae,
-                                    F(kMinInvDepth), F(kMaxInvDepth), result_idep, result_var);
+  const float err = search_point<I>(J, x, y, epi, gradient_max, gae, F(kMinInvDepth),
+                                    F(kMaxInvDepth), result_idep, result_var);
   const F diff = result_idep - F(s.d.z);
   if (first_observe)
   {
@@ -577,7 +661,11 @@ __global__ void __launch_bounds__(kSdThreads, 4) k_sd_update(const __grid_consta
     {
       const F inc_var = F(s.d.y) * F(kSuccVarIncFac);
       const F new_var = (inc_var * result_var) / (inc_var + result_var);
-      const F new_idepth = (F(s.d.x) * result_var + result_idep * inc_var) / (inc_var + result_var);
+      // the reference build fuses the second product; spelled out, since the
+      // compiler's choice between the two depends on the code around them
+      const F num = I ? F(s.d.x) * result_var + result_idep * inc_var
+                      : F(__fmaf_rn(result_idep.v, inc_var.v, __fmul_rn(s.d.x, result_var.v)));
+      const F new_idepth = num / (inc_var + result_var);
       if (new_var < F(s.d.y))
         s.d.y = new_var.v;
       s.d.x = new_idepth.v;
@@ -825,13 +913,13 @@ __global__ void __launch_bounds__(kSdThreads)
 }
 
 template <bool I>
-void sd_sequence(const SdBatch &B, int blocks, cudaStream_t s)
+void sd_sequence(const SdBatch &B, int blocks, int tiles, cudaStream_t s)
 {
   k_sd_convert<<<blocks, kSdThreads, 0, s>>>(B);
   k_sd_init<<<blocks, kSdThreads, 0, s>>>(B);
   // update_keyframe (seed_matrix.cu:401-446): stereo update, hole filling,
   // regularisation, projection into the incoming frame
-  k_sd_update<I><<<blocks, kSdThreads, 0, s>>>(B);
+  k_sd_update<I><<<tiles, kSdThreads, 0, s>>>(B);
   k_sd_fill<I><<<blocks, kSdThreads, 0, s>>>(B, 0, kSdUpdate);
   k_sd_regularize<I><<<blocks, kSdThreads, 0, s>>>(B, 1, 0, kSdUpdate);
   k_sd_project<I><<<blocks, kSdThreads, 0, s>>>(B);
@@ -849,6 +937,14 @@ void sd_sequence(const SdBatch &B, int blocks, cudaStream_t s)
 } // namespace
 
 int sd_blocks(int W, int H) { return (W * H + kSdThreads - 1) / kSdThreads; }
+
+// Larger tiles fill the warps of the search better; a step of few pixels needs
+// the blocks more: below two waves of blocks (148 SMs x 4) the tiles are
+// halved (one 752x480 stream 122 us per step against 132 at 1024 pixels; nine
+// streams with 4.9 M pixels 836 us at 1024 against 874 at 512, 849 at 2048).
+int sd_tile(long pixels) { return pixels < 2L * 592 * kSdTile ? kSdTile / 2 : kSdTile; }
+
+int sd_tiles(int W, int H, int tile) { return (W * H + tile - 1) / tile; }
 
 void launch_u8_to_f32(const uint8_t *src, int W, int H, float *dst, size_t pitch,
                       cudaStream_t s)
@@ -888,14 +984,14 @@ cudaTextureObject_t sd_make_texture(const float *img, int W, int H, size_t pitch
   return t;
 }
 
-int launch_semidense(const SdBatch &B, int blocks, int ieee, cudaStream_t s)
+int launch_semidense(const SdBatch &B, int blocks, int tiles, int ieee, cudaStream_t s)
 {
   if (blocks <= 0)
     return 0;
   if (ieee)
-    sd_sequence<true>(B, blocks, s);
+    sd_sequence<true>(B, blocks, tiles, s);
   else
-    sd_sequence<false>(B, blocks, s);
+    sd_sequence<false>(B, blocks, tiles, s);
   return 12;
 }
 

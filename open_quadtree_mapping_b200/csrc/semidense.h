@@ -41,13 +41,19 @@ struct SdBatch
 {
   const SdJob *jobs; // device (null: the single job `one`)
   const int *prefix; // device: block prefix over the jobs (njobs + 1)
+  const int *tile_prefix; // ... of the stereo update's tiles, of `tile` pixels
+  int tile;
   int njobs;
   SdJob one;
 };
 
+// blocks of a W x H job: of the per-pixel kernels, and of the stereo update
 int sd_blocks(int W, int H);
-// enqueues the whole step sequence; returns the number of launches
-int launch_semidense(const SdBatch &B, int blocks, int ieee, cudaStream_t s);
+int sd_tile(long pixels); // pixels per block of the update, all streams' pixels given
+int sd_tiles(int W, int H, int tile);
+// enqueues the whole step sequence over the summed blocks and tiles; returns
+// the number of launches
+int launch_semidense(const SdBatch &B, int blocks, int tiles, int ieee, cudaStream_t s);
 // float copy of a u8 image (dense rows of W bytes) with row pitch `pitch`
 // floats
 void launch_u8_to_f32(const uint8_t *src, int W, int H, float *dst, size_t pitch,

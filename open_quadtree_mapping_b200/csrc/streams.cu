@@ -219,11 +219,11 @@ void StreamSet::set_semidense(bool on)
     {
       check(cudaHostAlloc((void **)&h_sdjobs_[q], sizeof(SdJob) * n, cudaHostAllocDefault),
             "pinned allocation");
-      check(cudaHostAlloc((void **)&h_sdprefix_[q], sizeof(int) * (n + 1), cudaHostAllocDefault),
+      check(cudaHostAlloc((void **)&h_sdprefix_[q], sizeof(int) * 2 * (n + 1), cudaHostAllocDefault),
             "pinned allocation");
     }
     check(cudaMalloc((void **)&d_sdjobs_, sizeof(SdJob) * n), "device allocation");
-    check(cudaMalloc((void **)&d_sdprefix_, sizeof(int) * (n + 1)), "device allocation");
+    check(cudaMalloc((void **)&d_sdprefix_, sizeof(int) * 2 * (n + 1)), "device allocation");
   }
   semidense_ = on;
   eng_->set_keep_sparse(on);
@@ -232,10 +232,15 @@ void StreamSet::set_semidense(bool on)
 void StreamSet::semidense_step(const std::vector<int> &which, int parity)
 {
   SdJob *jobs = h_sdjobs_[parity];
-  int *prefix = h_sdprefix_[parity];
+  // block prefix, then tile prefix, over the streams of the step
+  int *prefix = h_sdprefix_[parity], *tiles = prefix + which.size() + 1;
   const bool ieee = eng_->params().arith == QM_ARITH_IEEE;
+  long pixels = 0;
+  for (int i : which)
+    pixels += (long)st_[i].d.W * st_[i].d.H;
+  const int tile = sd_tile(pixels);
   int n = 0;
-  prefix[0] = 0;
+  prefix[0] = tiles[0] = 0;
   for (int i : which)
   {
     State &s = st_[i];
@@ -264,6 +269,7 @@ void StreamSet::semidense_step(const std::vector<int> &which, int parity)
     J.zkey = eng_->buffers(i).sdkey;
     std::memcpy(J.T, s.sd_T.d, sizeof(J.T));
     prefix[n + 1] = prefix[n] + sd_blocks(s.d.W, s.d.H);
+    tiles[n + 1] = tiles[n] + sd_tiles(s.d.W, s.d.H, tile);
     ++n;
     // the incoming image becomes the keyframe after a first frame or a switch
     if (s.sd_mode == kSdInit || s.sd_mode == kSdSwitch)
@@ -274,14 +280,16 @@ void StreamSet::semidense_step(const std::vector<int> &which, int parity)
   const cudaStream_t cs = eng_->stream();
   check(cudaMemcpyAsync(d_sdjobs_, jobs, sizeof(SdJob) * n, cudaMemcpyHostToDevice, cs),
         "semi-dense job upload");
-  check(cudaMemcpyAsync(d_sdprefix_, prefix, sizeof(int) * (n + 1), cudaMemcpyHostToDevice, cs),
+  check(cudaMemcpyAsync(d_sdprefix_, prefix, sizeof(int) * 2 * (n + 1), cudaMemcpyHostToDevice, cs),
         "semi-dense job upload");
   SdBatch B;
   std::memset(&B, 0, sizeof(B));
   B.jobs = d_sdjobs_;
   B.prefix = d_sdprefix_;
+  B.tile_prefix = d_sdprefix_ + n + 1;
+  B.tile = tile;
   B.njobs = n;
-  launch_semidense(B, prefix[n], ieee ? 1 : 0, cs);
+  launch_semidense(B, prefix[n], tiles[n], ieee ? 1 : 0, cs);
   check(cudaGetLastError(), "semi-dense launch");
 }
 
