@@ -198,7 +198,11 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
   // cells are few (and which have two or more half-sweeps) run as one cluster
   // launch; below them each level runs job range by job range (message
   // inheritance, half-sweeps, and at level 0 the extraction)
+  // (a hypothesis count without jobs here has nothing to launch)
   std::vector<int> lc(T.dvals.size(), L);
+  auto any_of = [&](int d, int j0, int j1) {
+    return std::find(T.job_d.begin() + j0, T.job_d.begin() + j1, d) != T.job_d.begin() + j1;
+  };
   for (size_t di = 0; coarse_cells > 0 && di < T.dvals.size(); ++di)
   {
     const int d = T.dvals[di];
@@ -247,7 +251,7 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
           {
             b.rev = it & 1;
             for (size_t di = 0; di < T.dvals.size(); ++di)
-              if (l < lc[di])
+              if (l < lc[di] && any_of(T.dvals[di], j0, j1))
                 launch(kSweep, [&] {
                   launch_bp_sweep(b, grid, T.dvals[di], l, it, kp, ar, s, T.tune.sweep_warps,
                                   fold && in(st.inherit(l)) ? 1 : 0);
@@ -261,6 +265,8 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
         if (grid > 0)
           for (size_t di = 0; di < T.dvals.size(); ++di)
           {
+            if (!any_of(T.dvals[di], j0, j1))
+              continue;
             b.rev = (lc[di] > 0 && p.bp_iters[0] > 0) ? 1 - ((p.bp_iters[0] - 1) & 1) : 0;
             launch(kExtract,
                    [&] { launch_extract(b, grid, T.dvals[di], ar, s, T.tune.extract_warps); });
@@ -476,7 +482,8 @@ struct TableBuf
 
 struct Plan
 {
-  std::vector<int> active;
+  std::vector<int> active; // in launch order: streams of one hypothesis count together
+  std::vector<int> cuts;   // branch i runs jobs [cuts[i], cuts[i + 1]) of it
   std::unique_ptr<TableBuf> tb;
   bool tuned = false;                  // launch shapes settled (timed or fixed)
   size_t group_bytes = 0;              // the job grouping the graphs were captured with
@@ -725,6 +732,52 @@ std::unique_ptr<TableBuf> Engine::build_table(const std::vector<int> &active, co
   return tb;
 }
 
+// Branch boundaries of the jobs `order` (sorted by hypothesis count).  One
+// count: `branches_` equal ranges.  Several: the BP and the extraction launch
+// once per count, one after the other within a branch, so each count gets a
+// branch of its own (branches_ >= 2, at most kMaxBranches), and a range with
+// more than its share of the work (pixels times hypotheses over branches_) is
+// halved while branches are left.  Dense pass of mixed streams, two equal
+// ranges before: nine of 48, 64 and 96 hypotheses 1.65 -> 1.30 ms, sixteen
+// 2.6 -> 1.91 (a fourth branch whatever the shares: 1.31 and 1.91).
+std::vector<int> Engine::branch_cuts(const std::vector<int> &order) const
+{
+  const int n = (int)order.size();
+  std::vector<int> cuts{0};
+  if (branches_ >= 2)
+    for (int i = 1; i < n && (int)cuts.size() < kMaxBranches; ++i)
+      if (shapes_[order[i]].D != shapes_[order[i - 1]].D)
+        cuts.push_back(i);
+  if (cuts.size() == 1)
+  {
+    const int k = std::min(branches_, n);
+    for (int i = 1; i <= k; ++i)
+      cuts.push_back(n * i / k);
+    return cuts;
+  }
+  cuts.push_back(n);
+  auto work = [&](int i) {
+    double s = 0.0;
+    for (int j = cuts[i]; j < cuts[i + 1]; ++j)
+      s += (double)shapes_[order[j]].W * shapes_[order[j]].H * shapes_[order[j]].D;
+    return s;
+  };
+  double share = 0.0;
+  for (int i = 0; i + 1 < (int)cuts.size(); ++i)
+    share += work(i) / branches_;
+  while ((int)cuts.size() - 1 < kMaxBranches)
+  {
+    int best = -1;
+    for (int i = 0; i + 1 < (int)cuts.size(); ++i)
+      if (cuts[i + 1] - cuts[i] > 1 && (best < 0 || work(i) > work(best)))
+        best = i;
+    if (best < 0 || work(best) <= share)
+      break;
+    cuts.insert(cuts.begin() + best + 1, (cuts[best] + cuts[best + 1]) / 2);
+  }
+  return cuts;
+}
+
 Plan &Engine::plan_for(const std::vector<int> &active)
 {
   auto it = plans_.find(active);
@@ -738,6 +791,9 @@ Plan &Engine::plan_for(const std::vector<int> &active)
   }
   auto pl = std::make_unique<Plan>();
   pl->active = active;
+  std::stable_sort(pl->active.begin(), pl->active.end(),
+                   [&](int a, int b) { return shapes_[a].D < shapes_[b].D; });
+  pl->cuts = branch_cuts(pl->active);
   int max_w = 0, max_h = 0;
   for (int j : active)
   {
@@ -749,7 +805,7 @@ Plan &Engine::plan_for(const std::vector<int> &active)
   Tune t = fixed_tune_;
   if (!validate(t, max_w, max_h).empty())
     t = Tune{};
-  pl->tb = build_table(active, t);
+  pl->tb = build_table(pl->active, t);
   pl->tuned = !autotune_;
   Plan &ref = *pl;
   plans_[active] = std::move(pl);
@@ -925,8 +981,7 @@ int Engine::enqueue(Plan &pl, cudaStream_t s)
   pl.group_bytes = group_bytes_;
   pl.coarse_cells = coarse_cells_;
   pl.stagger = stagger_;
-  const int n = (int)pl.active.size();
-  const int k = std::min(branches_, n);
+  const int k = (int)pl.cuts.size() - 1;
   if (k < 2)
     return enqueue_range(B, pl.table(), params_, group_bytes_, coarse_cells_, 0, st.count() - 1,
                          s);
@@ -942,7 +997,7 @@ int Engine::enqueue(Plan &pl, cudaStream_t s)
   for (int i = 0; i < k; ++i)
   {
     cudaStream_t bs = i == 0 ? s : branch_[i - 1];
-    const int ja = n * i / k, jb = n * (i + 1) / k;
+    const int ja = pl.cuts[i], jb = pl.cuts[i + 1];
     if (i > 0)
       check(cudaStreamWaitEvent(bs, stagger_ ? ev_stage_[i - 1] : ev_fork_, 0), "fork");
     if (stagger_ && i + 1 < k)
@@ -977,7 +1032,7 @@ void Engine::launch(const std::vector<int> &active)
     return;
   check(cudaSetDevice(device_), "cudaSetDevice");
   Plan &pl = plan_for(active);
-  pack(active);
+  pack(pl.active);
   if (!pl.tuned)
     tune_plan(pl);
   last_tune_ = pl.table().tune;
@@ -1033,7 +1088,7 @@ void Engine::profile(const std::vector<int> &active, float *ms, int *launches)
 {
   check(cudaSetDevice(device_), "cudaSetDevice");
   Plan &pl = plan_for(active);
-  pack(active);
+  pack(pl.active);
   if (!pl.tuned)
     tune_plan(pl);
   last_tune_ = pl.table().tune;

@@ -228,6 +228,7 @@ public:
 
 private:
   Plan &plan_for(const std::vector<int> &active);
+  std::vector<int> branch_cuts(const std::vector<int> &order) const;
   std::unique_ptr<TableBuf> build_table(const std::vector<int> &active, const Tune &tune);
   void tune_plan(Plan &pl);
   // packs the descriptors of `active` into the pinned run array
