@@ -199,7 +199,7 @@ int qm_batch_set_semidense(qm_batch *b, int enable);
 /* k = 1..4 concurrent branches of the dense pipeline over consecutive
  * ranges of the streams that step together (the GPU fills one branch's
  * latency-bound stages -- coarse BP levels, line solves -- with the others'
- * work); 1 = one sequence over all of them; default 2.  With k >= 2 streams
+ * work); 1 = one sequence over all of them; default 3.  With k >= 2 streams
  * of different hypothesis counts get branches of their own, up to 4 in all.
  * Results do not depend on it. */
 int qm_batch_set_branches(qm_batch *b, int branches);

@@ -489,16 +489,20 @@ struct Plan
   size_t group_bytes = 0;              // the job grouping the graphs were captured with
   int coarse_cells = 0;                // the coarse-level threshold they were captured with
   bool stagger = false;                // the branch staggering they were captured with
-  cudaGraphExec_t exec[2] = {nullptr, nullptr}; // by step parity
+  // per branch; the second one is the rest of a staggered branch (the first
+  // ends with its cost volume)
+  cudaGraphExec_t exec[kMaxBranches][2] = {};
+  int launches[kMaxBranches][2] = {};
   StageTable &table() { return tb->table; }
   void drop_graphs()
   {
-    for (auto &e : exec)
-      if (e)
-      {
-        cudaGraphExecDestroy(e);
-        e = nullptr;
-      }
+    for (auto &b : exec)
+      for (auto &e : b)
+        if (e)
+        {
+          cudaGraphExecDestroy(e);
+          e = nullptr;
+        }
   }
   ~Plan() { drop_graphs(); }
 };
@@ -533,14 +537,28 @@ Engine::Engine(int device, const qm_params &p, const std::vector<Shape> &shapes)
       throw CudaError{QM_ERR_INVALID_ARG, err};
   }
   check(cudaSetDevice(device), "cudaSetDevice");
-  check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
+  // Branch i before branch i + 1, the last one at the default priority: the
+  // branches drift apart, so that the cost kernel of one (bound by instruction
+  // issue) runs beside the BP of another (bound by HBM), and the first branch's
+  // results leave while the others still compute.  Measured with three
+  // branches, equal priorities -> these: 32 x 752x480 submit + wait 3.98 ->
+  // 3.32 ms, resident 2.53 -> 2.50; 8 x 1920x1080 10.3 -> 9.5, 8.98 -> 8.88.
+  int low = 0, high = 0;
+  check(cudaDeviceGetStreamPriorityRange(&low, &high), "stream priorities");
+  auto make = [&](cudaStream_t *s, int i) {
+    check(cudaStreamCreateWithPriority(s, cudaStreamNonBlocking,
+                                       std::max(high, low - (kMaxBranches - 1 - i))),
+          "cudaStreamCreate");
+  };
+  make(&stream_, 0);
   check(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming), "cudaEventCreate");
   for (int i = 0; i + 1 < kMaxBranches; ++i)
   {
-    check(cudaStreamCreateWithFlags(&branch_[i], cudaStreamNonBlocking), "cudaStreamCreate");
-    check(cudaEventCreateWithFlags(&ev_join_[i], cudaEventDisableTiming), "cudaEventCreate");
+    make(&branch_[i], i + 1);
     check(cudaEventCreateWithFlags(&ev_stage_[i], cudaEventDisableTiming), "cudaEventCreate");
   }
+  for (auto &e : ev_branch_)
+    check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
   check(cudaEventCreate(&ev0_), "cudaEventCreate");
   check(cudaEventCreate(&ev1_), "cudaEventCreate");
   prepare_upsample_kernels();
@@ -597,32 +615,30 @@ Engine::Engine(int device, const qm_params &p, const std::vector<Shape> &shapes)
     slot_base_[j] = total_slots_;
     total_slots_ += shapes[j].F;
   }
-  for (int q = 0; q < 2; ++q)
+  const size_t o_ptr = align256(sizeof(JobDesc) * n);
+  const size_t o_T = o_ptr + align256(sizeof(void *) * total_slots_);
+  const size_t o_w = o_T + align256(sizeof(float) * 12 * total_slots_);
+  block_bytes_ = o_w + sizeof(int) * total_slots_;
+  auto cut = [&](char *base) {
+    return StepBlock{base, (JobDesc *)base, (const uint8_t **)(base + o_ptr),
+                     (float *)(base + o_T), (int *)(base + o_w)};
+  };
+  for (auto &h : h_block_)
   {
-    check(cudaHostAlloc((void **)&h_slot_ptr_[q], sizeof(void *) * total_slots_,
-                        cudaHostAllocDefault),
-          "pinned allocation");
-    check(cudaHostAlloc((void **)&h_slot_T_[q], sizeof(float) * 12 * total_slots_,
-                        cudaHostAllocDefault),
-          "pinned allocation");
-    check(cudaHostAlloc((void **)&h_slot_w_[q], sizeof(int) * total_slots_, cudaHostAllocDefault),
-          "pinned allocation");
-    std::memset(h_slot_ptr_[q], 0, sizeof(void *) * total_slots_);
-    std::memset(h_slot_T_[q], 0, sizeof(float) * 12 * total_slots_);
-    std::memset(h_slot_w_[q], 0, sizeof(int) * total_slots_);
-    check(cudaHostAlloc((void **)&h_run_[q], sizeof(JobDesc) * n, cudaHostAllocDefault),
-          "pinned allocation");
+    char *base = nullptr;
+    check(cudaHostAlloc((void **)&base, block_bytes_, cudaHostAllocDefault), "pinned allocation");
+    std::memset(base, 0, block_bytes_);
+    h = cut(base);
   }
-  check(cudaMalloc((void **)&d_slot_ptr_, sizeof(void *) * total_slots_), "device allocation");
-  check(cudaMalloc((void **)&d_slot_T_, sizeof(float) * 12 * total_slots_), "device allocation");
-  check(cudaMalloc((void **)&d_slot_w_, sizeof(int) * total_slots_), "device allocation");
+  char *dev_base = nullptr;
+  check(cudaMalloc((void **)&dev_base, block_bytes_), "device allocation");
+  d_block_ = cut(dev_base);
   master_.resize(n);
   for (int j = 0; j < n; ++j)
   {
     master_[j] = make_job_desc(shapes[j], p, bufs_[j], 0);
     master_[j].slot_base = slot_base_[j];
   }
-  check(cudaMalloc((void **)&d_run_, sizeof(JobDesc) * n), "device allocation");
   check(cudaStreamSynchronize(stream_), "engine init");
 }
 
@@ -634,25 +650,11 @@ Engine::~Engine()
   plans_.clear();
   if (arena_)
     cudaFree(arena_);
-  if (d_slot_ptr_)
-    cudaFree(d_slot_ptr_);
-  if (d_slot_T_)
-    cudaFree(d_slot_T_);
-  if (d_slot_w_)
-    cudaFree(d_slot_w_);
-  if (d_run_)
-    cudaFree(d_run_);
-  for (int q = 0; q < 2; ++q)
-  {
-    if (h_slot_ptr_[q])
-      cudaFreeHost(h_slot_ptr_[q]);
-    if (h_slot_T_[q])
-      cudaFreeHost(h_slot_T_[q]);
-    if (h_slot_w_[q])
-      cudaFreeHost(h_slot_w_[q]);
-    if (h_run_[q])
-      cudaFreeHost(h_run_[q]);
-  }
+  if (d_block_.base)
+    cudaFree(d_block_.base);
+  for (auto &h : h_block_)
+    if (h.base)
+      cudaFreeHost(h.base);
   if (ev0_)
     cudaEventDestroy(ev0_);
   if (ev1_)
@@ -664,11 +666,12 @@ Engine::~Engine()
       cudaStreamSynchronize(branch_[i]);
       cudaStreamDestroy(branch_[i]);
     }
-    if (ev_join_[i])
-      cudaEventDestroy(ev_join_[i]);
     if (ev_stage_[i])
       cudaEventDestroy(ev_stage_[i]);
   }
+  for (auto &e : ev_branch_)
+    if (e)
+      cudaEventDestroy(e);
   if (ev_fork_)
     cudaEventDestroy(ev_fork_);
   if (stream_)
@@ -684,8 +687,9 @@ void Engine::set_inputs(int j, const uint8_t *ref, int ref_pitch, const uint8_t 
   J.slot_pitch = slot_pitch;
   const int b = slot_base_[j];
   const int q = parity_;
-  J.F = dedupe_slots(shapes_[j].F, slots, T_slot_ref, h_slot_ptr_[q] + b, h_slot_T_[q] + 12 * b,
-                     h_slot_w_[q] + b);
+  const StepBlock &h = h_block_[q];
+  J.F = dedupe_slots(shapes_[j].F, slots, T_slot_ref, h.slot_ptr + b, h.slot_T + 12 * b,
+                     h.slot_w + b);
   if (T_fuse)
     std::memcpy(J.Tf, T_fuse, 12 * sizeof(float));
 }
@@ -946,78 +950,66 @@ void Engine::pack(const std::vector<int> &active)
     J.seeds_in = bufs_[j].seeds[seeds_cur_[j]];
     J.seeds_out = bufs_[j].seeds[seeds_cur_[j] ^ 1];
     J.dense = bufs_[j].dense[parity_];
-    h_run_[parity_][i] = J;
+    h_block_[parity_].run[i] = J;
   }
 }
 
 Batch Engine::upload(int n, cudaStream_t s)
 {
-  const int q = parity_;
-  check(cudaMemcpyAsync(d_run_, h_run_[q], sizeof(JobDesc) * n, cudaMemcpyHostToDevice, s),
+  check(cudaMemcpyAsync(d_block_.base, h_block_[parity_].base, block_bytes_,
+                        cudaMemcpyHostToDevice, s),
         "descriptor upload");
-  check(cudaMemcpyAsync(d_slot_ptr_, h_slot_ptr_[q], sizeof(void *) * total_slots_,
-                        cudaMemcpyHostToDevice, s),
-        "slot upload");
-  check(cudaMemcpyAsync(d_slot_T_, h_slot_T_[q], sizeof(float) * 12 * total_slots_,
-                        cudaMemcpyHostToDevice, s),
-        "slot upload");
-  check(cudaMemcpyAsync(d_slot_w_, h_slot_w_[q], sizeof(int) * total_slots_,
-                        cudaMemcpyHostToDevice, s),
-        "slot upload");
   Batch B;
   std::memset(&B, 0, sizeof(B));
-  B.jobs = d_run_;
+  B.jobs = d_block_.run;
   B.njobs = n;
-  B.slot_ptr = d_slot_ptr_;
-  B.slot_T = d_slot_T_;
-  B.slot_w = d_slot_w_;
+  B.slot_ptr = d_block_.slot_ptr;
+  B.slot_T = d_block_.slot_T;
+  B.slot_w = d_block_.slot_w;
   return B;
 }
 
-int Engine::enqueue(Plan &pl, cudaStream_t s)
+void Engine::run_part(Plan &pl, const Batch &B, int i, int part, int first, int last,
+                      cudaStream_t s)
 {
-  const Batch B = upload((int)pl.active.size(), s);
-  const Stages st{params_.bp_levels};
-  pl.group_bytes = group_bytes_;
-  pl.coarse_cells = coarse_cells_;
-  pl.stagger = stagger_;
-  const int k = (int)pl.cuts.size() - 1;
-  if (k < 2)
-    return enqueue_range(B, pl.table(), params_, group_bytes_, coarse_cells_, 0, st.count() - 1,
-                         s);
-  // k independent branches over consecutive ranges of the jobs (every stage
-  // is per job): the GPU fills the latency-bound stretches of one branch
-  // (coarse BP levels, line solves) with the other branches' work
-  // Staggered (optional): branch i + 1 starts when branch i's cost volume
-  // is done, so that cost kernels (bound by instruction issue) run beside
-  // the previous branch's BP half-sweeps (bound by HBM bandwidth) instead of
-  // beside each other.
-  check(cudaEventRecord(ev_fork_, s), "fork");
-  int nl = 0;
-  for (int i = 0; i < k; ++i)
+  const int ja = pl.cuts[i], jb = pl.cuts[i + 1];
+  if (!graphs_)
   {
-    cudaStream_t bs = i == 0 ? s : branch_[i - 1];
-    const int ja = pl.cuts[i], jb = pl.cuts[i + 1];
-    if (i > 0)
-      check(cudaStreamWaitEvent(bs, stagger_ ? ev_stage_[i - 1] : ev_fork_, 0), "fork");
-    if (stagger_ && i + 1 < k)
+    pl.launches[i][part] = enqueue_range(B, pl.table(), params_, group_bytes_, coarse_cells_,
+                                         first, last, s, nullptr, ja, jb);
+    return;
+  }
+  cudaGraphExec_t &exec = pl.exec[i][part];
+  if (!exec)
+  {
+    cudaGraph_t g = nullptr;
+    check(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "graph capture");
+    try
     {
-      nl += enqueue_range(B, pl.table(), params_, group_bytes_, coarse_cells_, 0, st.cost(), bs,
-                          nullptr, ja, jb);
-      check(cudaEventRecord(ev_stage_[i], bs), "stage");
-      nl += enqueue_range(B, pl.table(), params_, group_bytes_, coarse_cells_, st.cost() + 1,
-                          st.count() - 1, bs, nullptr, ja, jb);
+      pl.launches[i][part] = enqueue_range(B, pl.table(), params_, group_bytes_, coarse_cells_,
+                                           first, last, s, nullptr, ja, jb);
     }
-    else
-      nl += enqueue_range(B, pl.table(), params_, group_bytes_, coarse_cells_, 0, st.count() - 1,
-                          bs, nullptr, ja, jb);
+    catch (...)
+    {
+      cudaStreamEndCapture(s, &g);
+      if (g)
+        cudaGraphDestroy(g);
+      throw;
+    }
+    check(cudaStreamEndCapture(s, &g), "graph capture");
+    const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
+    cudaGraphDestroy(g);
+    check(e, "graph instantiate");
   }
-  for (int i = 1; i < k; ++i)
-  {
-    check(cudaEventRecord(ev_join_[i - 1], branch_[i - 1]), "join");
-    check(cudaStreamWaitEvent(s, ev_join_[i - 1], 0), "join");
-  }
-  return nl;
+  check(cudaGraphLaunch(exec, s), "graph launch");
+}
+
+void Engine::layout(const std::vector<int> &active, std::vector<int> &order,
+                    std::vector<int> &cuts)
+{
+  const Plan &pl = plan_for(active);
+  order = pl.active;
+  cuts = pl.cuts;
 }
 
 void Engine::run(const std::vector<int> &active)
@@ -1026,53 +1018,64 @@ void Engine::run(const std::vector<int> &active)
   check(cudaStreamSynchronize(stream_), "pipeline run");
 }
 
-void Engine::launch(const std::vector<int> &active)
+// The descriptors go up first, in one copy; then every branch runs its own
+// graph on its own stream, so that a branch starts when its own inputs are
+// there (ready) and its results can leave when it is done, while the other
+// branches still run.  A branch is a consecutive range of jobs, which share
+// nothing: the GPU fills the latency-bound stretches of one with the others'
+// work.  The graphs read the descriptors from one device block, so they serve
+// every step.
+// Staggered (optional): branch i + 1 starts when branch i's cost volume is
+// done, so that cost kernels (bound by instruction issue) run beside the
+// previous branch's BP half-sweeps (bound by HBM bandwidth).
+void Engine::launch(const std::vector<int> &active, const cudaEvent_t *ready)
 {
   if (active.empty())
     return;
   check(cudaSetDevice(device_), "cudaSetDevice");
   Plan &pl = plan_for(active);
   pack(pl.active);
+  const int k = (int)pl.cuts.size() - 1;
   if (!pl.tuned)
+  {
+    for (int i = 0; ready && i < k; ++i)
+      check(cudaStreamWaitEvent(stream_, ready[i], 0), "inputs");
     tune_plan(pl);
+  }
   last_tune_ = pl.table().tune;
-  if (graphs_)
+  pl.group_bytes = group_bytes_;
+  pl.coarse_cells = coarse_cells_;
+  pl.stagger = stagger_;
+  const Stages st{params_.bp_levels};
+  check(cudaEventRecord(ev0_, stream_), "event");
+  const Batch B = upload((int)pl.active.size(), stream_);
+  if (k > 1)
+    check(cudaEventRecord(ev_fork_, stream_), "fork");
+  for (int i = 0; i < k; ++i)
   {
-    // one graph per parity: its memcpy nodes read that parity's pinned
-    // descriptor and slot tables
-    cudaGraphExec_t &exec = pl.exec[parity_];
-    if (!exec)
+    cudaStream_t s = i == 0 ? stream_ : branch_[i - 1];
+    if (i > 0)
+      check(cudaStreamWaitEvent(s, ev_fork_, 0), "fork");
+    if (ready)
+      check(cudaStreamWaitEvent(s, ready[i], 0), "inputs");
+    if (i > 0 && stagger_)
+      check(cudaStreamWaitEvent(s, ev_stage_[i - 1], 0), "stage");
+    if (stagger_ && i + 1 < k)
     {
-      cudaGraph_t g = nullptr;
-      check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "graph capture");
-      int nl = 0;
-      try
-      {
-        nl = enqueue(pl, stream_);
-      }
-      catch (...)
-      {
-        cudaStreamEndCapture(stream_, &g);
-        if (g)
-          cudaGraphDestroy(g);
-        throw;
-      }
-      check(cudaStreamEndCapture(stream_, &g), "graph capture");
-      const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
-      cudaGraphDestroy(g);
-      check(e, "graph instantiate");
-      last_launches_ = nl;
+      run_part(pl, B, i, 0, 0, st.cost(), s);
+      check(cudaEventRecord(ev_stage_[i], s), "stage");
+      run_part(pl, B, i, 1, st.cost() + 1, st.count() - 1, s);
     }
-    check(cudaEventRecord(ev0_, stream_), "event");
-    check(cudaGraphLaunch(exec, stream_), "graph launch");
-    check(cudaEventRecord(ev1_, stream_), "event");
+    else
+      run_part(pl, B, i, 0, 0, st.count() - 1, s);
+    check(cudaEventRecord(ev_branch_[i], s), "branch");
   }
-  else
-  {
-    check(cudaEventRecord(ev0_, stream_), "event");
-    last_launches_ = enqueue(pl, stream_);
-    check(cudaEventRecord(ev1_, stream_), "event");
-  }
+  for (int i = 1; i < k; ++i)
+    check(cudaStreamWaitEvent(stream_, ev_branch_[i], 0), "join");
+  check(cudaEventRecord(ev1_, stream_), "event");
+  last_launches_ = 0;
+  for (int i = 0; i < k; ++i)
+    last_launches_ += pl.launches[i][0] + (stagger_ && i + 1 < k ? pl.launches[i][1] : 0);
   for (int j : active)
     seeds_cur_[j] ^= 1;
 }

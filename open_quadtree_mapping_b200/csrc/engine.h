@@ -55,10 +55,6 @@ enum KernelKind
 // 5.23 ms at 24 MiB).
 constexpr size_t kDefaultGroupBytes = 0;
 
-// Default number of concurrent pipeline branches per batch: two (the halves
-// of the active jobs as independent graph branches) measured 3 % faster than
-// one sequence at 32 streams of 752x480 (3.27 vs 3.37 ms per batch), with
-// bit-identical results.
 // Default coarse-level threshold of the BP: the top pyramid levels whose
 // largest cell count over the active jobs is at most this run all their
 // half-sweeps in one cluster launch (k_bp_coarse) instead of one launch per
@@ -69,8 +65,13 @@ constexpr size_t kDefaultGroupBytes = 0;
 #define QM_DEFAULT_COARSE_CELLS 4096
 #endif
 
+// Default number of concurrent pipeline branches per batch (consecutive ranges
+// of the active jobs, bit-identical results).  submit + wait / resident, two
+// and three branches: 32 x 752x480 3.45 / 2.48 and 3.32 / 2.50 ms, 8 x 752x480
+// 0.96 / 0.73 and 0.92 / 0.72, 8 x 1920x1080 9.73 / 8.93 and 9.47 / 8.88; four:
+// 3.34 / 2.61 and 9.24 / 8.82.
 #ifndef QM_DEFAULT_BRANCHES
-#define QM_DEFAULT_BRANCHES 2
+#define QM_DEFAULT_BRANCHES 3
 #endif
 constexpr int kMaxBranches = 4;
 
@@ -176,9 +177,15 @@ public:
   float4 *seeds(int j) const { return bufs_[j].seeds[seeds_cur_[j]]; }
   void reset_seeds(int j);
 
-  // Enqueues the pipeline for `active` job indices on stream() without
-  // waiting.  Throws CudaError.  Graph capture is used when `graphs` is set.
-  void launch(const std::vector<int> &active);
+  // Enqueues the pipeline for `active` job indices without waiting; stream()
+  // is behind it.  Throws CudaError.  Graph capture is used when `graphs` is
+  // set.  ready[i] (may be null): event branch i waits for before it starts.
+  void launch(const std::vector<int> &active, const cudaEvent_t *ready = nullptr);
+  // The branches of the next launch of `active`: branch i runs the jobs
+  // order[cuts[i]] .. order[cuts[i + 1] - 1].  After the launch,
+  // branch_done(i) marks its end.
+  void layout(const std::vector<int> &active, std::vector<int> &order, std::vector<int> &cuts);
+  cudaEvent_t branch_done(int i) const { return ev_branch_[i]; }
   // launch() and wait for it
   void run(const std::vector<int> &active);
   void set_graphs(bool on) { graphs_ = on; }
@@ -235,7 +242,9 @@ private:
   void pack(const std::vector<int> &active);
   // enqueues the descriptor and slot-table uploads; returns the batch
   Batch upload(int n, cudaStream_t s);
-  int enqueue(Plan &pl, cudaStream_t s);
+  // runs stages [first, last] of branch i on s, from its graph when graphs are
+  // on (part: which of the plan's graphs)
+  void run_part(Plan &pl, const Batch &B, int i, int part, int first, int last, cudaStream_t s);
 
   int device_;
   qm_params params_;
@@ -244,22 +253,25 @@ private:
   std::vector<JobBuffers> bufs_;
   std::vector<int> seeds_cur_;
   void *arena_ = nullptr;
-  // slot tables (all jobs), pinned host + device
+  // One step's descriptors -- the packed job descriptors, then the slot tables
+  // of all jobs (image, pose, multiplicity) -- as one block: pinned per parity,
+  // and its device copy
   std::vector<int> slot_base_;
   int total_slots_ = 0;
-  const uint8_t **h_slot_ptr_[2] = {};
-  float *h_slot_T_[2] = {};
-  int *h_slot_w_[2] = {};
-  const uint8_t **d_slot_ptr_ = nullptr;
-  float *d_slot_T_ = nullptr;
-  int *d_slot_w_ = nullptr;
-  // job descriptors: host master copy and the packed run arrays
-  std::vector<JobDesc> master_;
-  JobDesc *h_run_[2] = {};
-  JobDesc *d_run_ = nullptr;
+  struct StepBlock
+  {
+    char *base = nullptr;
+    JobDesc *run = nullptr;
+    const uint8_t **slot_ptr = nullptr;
+    float *slot_T = nullptr;
+    int *slot_w = nullptr;
+  };
+  size_t block_bytes_ = 0;
+  StepBlock h_block_[2], d_block_;
+  std::vector<JobDesc> master_; // host master copies of the descriptors
   cudaStream_t stream_ = nullptr;
   cudaStream_t branch_[kMaxBranches - 1] = {}; // streams of branches 2..k
-  cudaEvent_t ev_fork_ = nullptr, ev_join_[kMaxBranches - 1] = {};
+  cudaEvent_t ev_fork_ = nullptr, ev_branch_[kMaxBranches] = {}; // branch i done
   cudaEvent_t ev_stage_[kMaxBranches - 1] = {}; // branch i's cost stage done
   bool stagger_ = false;
   int branches_ = QM_DEFAULT_BRANCHES;

@@ -75,6 +75,12 @@ SE3f operator*(const SE3f &lhs, const SE3f &rhs)
 namespace
 {
 constexpr int kRing = QM_RING_CAPACITY;
+// frames of a stream's pool.  In use at most: the ring, the image of the last
+// result (when it did not join the ring), the incoming frame, and what the
+// step before freed, which becomes free when that step has retired (a frame
+// that left the ring and the previous result's image; both only when its own
+// incoming frame joined the ring, which then is the last result's image).
+constexpr int kPoolFrames = kRing + 3;
 
 float dot3(const float *a, const float *b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
 
@@ -122,16 +128,18 @@ StreamSet::StreamSet(int device, const qm_params &p, const std::vector<StreamDes
     check(cudaEventCreateWithFlags(&ev_comp_[q], cudaEventDisableTiming), "cudaEventCreate");
     check(cudaEventCreateWithFlags(&ev_done_[q], cudaEventDisableTiming), "cudaEventCreate");
   }
+  for (auto &e : ev_in_)
+    check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
   st_.resize(descs.size());
   for (size_t i = 0; i < descs.size(); ++i)
   {
     State &s = st_[i];
     s.d = descs[i];
     const size_t frame = (size_t)s.d.W * s.d.H;
-    // ring + income + spare frames, and the image of the last result
-    check(cudaMalloc((void **)&s.pool, frame * (kRing + 3)), "frame pool allocation");
-    for (int k = kRing + 1; k >= 0; --k)
+    check(cudaMalloc((void **)&s.pool, frame * kPoolFrames), "frame pool allocation");
+    for (int k = kPoolFrames - 1; k >= 0; --k)
       s.free_slots.push_back(k);
+    s.held.assign(kPoolFrames, 0);
     s.income_T = s.keyframe_T = s.fuse_T = s.T_world_ref = SE3f::identity();
   }
 }
@@ -153,6 +161,9 @@ StreamSet::~StreamSet()
     if (ev_done_[q])
       cudaEventDestroy(ev_done_[q]);
   }
+  for (auto &e : ev_in_)
+    if (e)
+      cudaEventDestroy(e);
   if (up_)
     cudaStreamDestroy(up_);
   if (down_)
@@ -305,26 +316,36 @@ bool StreamSet::need_switch_keyframe(const State &s) const
   return moved(s.keyframe_T, s.income_T, 0.86, 0.5);
 }
 
-StreamSet::Outcome StreamSet::begin_frame(int i, const uint8_t *img, size_t stride,
-                                          const float *T)
+// a dense image goes up as one linear copy (row-by-row 2D copies of short rows
+// are much slower on the copy engines)
+void StreamSet::upload(int i, const uint8_t *img, size_t stride)
+{
+  const State &s = st_[i];
+  const size_t W = s.d.W, H = s.d.H;
+  uint8_t *to = frame_ptr(s, s.income_slot);
+  if (stride == W)
+    check(cudaMemcpyAsync(to, img, W * H, cudaMemcpyHostToDevice, up_), "image upload");
+  else
+    check(cudaMemcpy2DAsync(to, W, img, stride, W, H, cudaMemcpyHostToDevice, up_),
+          "image upload");
+}
+
+// one holder of a frame slot lets go; the last one's step may still read it,
+// so it becomes free once that step has retired
+void StreamSet::release(int i, int slot, int parity)
+{
+  if (--st_[i].held[slot] == 0)
+    pending_[parity].push_back({i, slot});
+}
+
+StreamSet::Outcome StreamSet::begin_frame(int i, const float *T)
 {
   State &s = st_[i];
-  const int W = s.d.W, H = s.d.H;
-  if (!img || !T || stride < (size_t)W)
-    throw CudaError{QM_ERR_INVALID_ARG, "image pointer, stride or pose invalid"};
+  const int W = s.d.W;
   s.frame_index++;
   s.income_slot = s.free_slots.back();
   s.free_slots.pop_back();
-  // a dense image goes up as one linear copy (row-by-row 2D copies of short
-  // rows are much slower on the copy engines)
-  if (stride == (size_t)W)
-    check(cudaMemcpyAsync(frame_ptr(s, s.income_slot), img, (size_t)W * H,
-                          cudaMemcpyHostToDevice, up_),
-          "image upload");
-  else
-    check(cudaMemcpy2DAsync(frame_ptr(s, s.income_slot), W, img, stride, W, H,
-                            cudaMemcpyHostToDevice, up_),
-          "image upload");
+  s.held[s.income_slot] = 1;
   s.income_T = SE3f::from(T);
   if (!s.initialized)
   {
@@ -366,28 +387,27 @@ StreamSet::Outcome StreamSet::begin_frame(int i, const uint8_t *img, size_t stri
   return kOutput;
 }
 
-// The image of the last result stays on the device (a copy into the pool's
-// last slot, ordered after the frame's upload on the engine stream) and is
-// only downloaded when asked for.
-void StreamSet::keep_reference(State &s)
+// The image of the last result stays on the device, in the slot it came in
+// with, and is only downloaded when asked for.
+void StreamSet::keep_reference(int i, int parity)
 {
-  check(cudaMemcpyAsync(ref_ptr(s), frame_ptr(s, s.income_slot), (size_t)s.d.W * s.d.H,
-                        cudaMemcpyDeviceToDevice, eng_->stream()),
-        "reference image copy");
-  s.has_ref = true;
+  State &s = st_[i];
+  if (s.ref_slot >= 0)
+    release(i, s.ref_slot, parity);
+  s.ref_slot = s.income_slot;
+  ++s.held[s.ref_slot];
 }
 
 void StreamSet::end_frame(int i, int parity)
 {
   State &s = st_[i];
   const size_t P = (size_t)s.d.W * s.d.H;
-  bool keep_income = false;
   if (s.outcome == kFirst)
   {
     const JobBuffers &b = eng_->buffers(i);
     check(cudaMemsetAsync(eng_->dense(i), 0, P * sizeof(float), eng_->stream()), "memset");
     check(cudaMemsetAsync(b.sparse, 0, P * sizeof(float), eng_->stream()), "memset");
-    keep_reference(s);
+    keep_reference(i, parity);
     s.T_world_ref = s.income_T.inv();
   }
   else if (s.outcome == kNoOutput || s.outcome == kOutput)
@@ -395,24 +415,21 @@ void StreamSet::end_frame(int i, int parity)
     if (need_add_reference(s))
     {
       s.ring.push_front(RingFrame{s.income_slot, s.income_T});
-      keep_income = true;
+      ++s.held[s.income_slot];
       if ((int)s.ring.size() > kRing)
       {
-        pending_[parity].push_back({i, s.ring.back().slot});
+        release(i, s.ring.back().slot, parity);
         s.ring.pop_back();
       }
     }
     if (s.outcome == kOutput)
     {
       s.fuse_T = s.income_T;
-      keep_reference(s);
+      keep_reference(i, parity);
       s.T_world_ref = s.income_T.inv();
     }
   }
-  // a freed slot may still be read by this step's pipeline: it becomes free
-  // again once the step has retired
-  if (!keep_income)
-    pending_[parity].push_back({i, s.income_slot});
+  release(i, s.income_slot, parity);
   s.income_slot = -1;
 }
 
@@ -462,23 +479,43 @@ void StreamSet::step(const std::vector<int> &which, const uint8_t *const *imgs,
     check(cudaEventSynchronize(ev_up_[p ^ 1]), "upload");
   eng_->set_parity(p);
   started_ = true;
-  std::vector<int> active;
+  std::vector<int> active, at(size(), -1); // at: position in `which`
   for (size_t k = 0; k < which.size(); ++k)
   {
     const int i = which[k];
-    st_[i].outcome = begin_frame(i, imgs[k], strides[k], T_curr_world + 12 * k);
+    at[i] = (int)k;
+    st_[i].outcome = begin_frame(i, T_curr_world + 12 * k);
     if (st_[i].outcome == kOutput)
       active.push_back(i);
   }
+  // Frames go up branch by branch, and a branch starts when its own are there;
+  // likewise its depth maps go down as soon as it is done, so that the copies
+  // of one branch run beside the kernels of the others also within one step.
+  std::vector<int> order, cuts{0};
+  if (!active.empty())
+    eng_->layout(active, order, cuts);
+  const int branches = (int)cuts.size() - 1;
+  for (int b = 0; b < branches; ++b)
+  {
+    for (int j = cuts[b]; j < cuts[b + 1]; ++j)
+      upload(order[j], imgs[at[order[j]]], strides[at[order[j]]]);
+    check(cudaEventRecord(ev_in_[b], up_), "event");
+  }
+  for (size_t k = 0; k < which.size(); ++k)
+    if (st_[which[k]].outcome != kOutput)
+      upload(which[k], imgs[k], strides[k]);
   check(cudaEventRecord(ev_up_[p], up_), "event");
-  check(cudaStreamWaitEvent(eng_->stream(), ev_up_[p], 0), "event wait");
   if (semidense_)
+  {
+    check(cudaStreamWaitEvent(eng_->stream(), ev_up_[p], 0), "event wait");
     semidense_step(which, p);
+  }
   if (!active.empty())
   {
-    eng_->launch(active);
+    eng_->launch(active, ev_in_);
     last_active_ = active;
   }
+  check(cudaStreamWaitEvent(eng_->stream(), ev_up_[p], 0), "event wait");
   for (size_t k = 0; k < which.size(); ++k)
   {
     end_frame(which[k], p);
@@ -488,25 +525,32 @@ void StreamSet::step(const std::vector<int> &which, const uint8_t *const *imgs,
       st_[which[k]].out_parity = p;
   }
   check(cudaEventRecord(ev_comp_[p], eng_->stream()), "event");
+  auto download = [&](int i) {
+    const int k = at[i];
+    if (!depth_outs || !has_result[k] || !depth_outs[k])
+      return;
+    const State &s = st_[i];
+    const float *src = eng_->dense(i);
+    const size_t stride = depth_strides ? depth_strides[k] : (size_t)s.d.W;
+    if (stride == (size_t)s.d.W)
+      check(cudaMemcpyAsync(depth_outs[k], src, sizeof(float) * s.d.W * s.d.H,
+                            cudaMemcpyDeviceToHost, down_),
+            "depth download");
+    else
+      check(cudaMemcpy2DAsync(depth_outs[k], stride * sizeof(float), src, s.d.W * sizeof(float),
+                              s.d.W * sizeof(float), s.d.H, cudaMemcpyDeviceToHost, down_),
+            "depth download");
+  };
+  for (int b = 0; b < branches; ++b)
+  {
+    check(cudaStreamWaitEvent(down_, eng_->branch_done(b), 0), "event wait");
+    for (int j = cuts[b]; j < cuts[b + 1]; ++j)
+      download(order[j]);
+  }
   check(cudaStreamWaitEvent(down_, ev_comp_[p], 0), "event wait");
-  if (depth_outs)
-    for (size_t k = 0; k < which.size(); ++k)
-    {
-      if (!has_result[k] || !depth_outs[k])
-        continue;
-      const State &s = st_[which[k]];
-      const float *src = eng_->dense(which[k]);
-      const size_t stride = depth_strides ? depth_strides[k] : (size_t)s.d.W;
-      if (stride == (size_t)s.d.W)
-        check(cudaMemcpyAsync(depth_outs[k], src, sizeof(float) * s.d.W * s.d.H,
-                              cudaMemcpyDeviceToHost, down_),
-              "depth download");
-      else
-        check(cudaMemcpy2DAsync(depth_outs[k], stride * sizeof(float), src,
-                                s.d.W * sizeof(float), s.d.W * sizeof(float), s.d.H,
-                                cudaMemcpyDeviceToHost, down_),
-              "depth download");
-    }
+  for (int i : which)
+    if (st_[i].outcome != kOutput)
+      download(i);
   check(cudaEventRecord(ev_done_[p], down_), "event");
   inflight_[p] = true;
   ++step_;
@@ -593,7 +637,7 @@ int StreamSet::get_point_cloud(int i, float *out, size_t capacity)
 {
   wait();
   const State &s = st_[i];
-  if (!s.has_ref)
+  if (s.ref_slot < 0)
     throw CudaError{QM_ERR_STATE, "no result yet"};
   const int W = s.d.W, H = s.d.H;
   // one device buffer for every stream: points of the largest image, the
@@ -660,7 +704,7 @@ void StreamSet::get_reference(int i, uint8_t *out, size_t stride)
 {
   wait();
   const State &s = st_[i];
-  if (!s.has_ref)
+  if (s.ref_slot < 0)
     throw CudaError{QM_ERR_STATE, "no result yet"};
   check(cudaMemcpy2D(out, stride, ref_ptr(s), s.d.W, s.d.W, s.d.H, cudaMemcpyDeviceToHost),
         "reference download");

@@ -100,7 +100,7 @@ private:
   struct State
   {
     StreamDesc d;
-    uint8_t *pool = nullptr; // (ring capacity + 2) frames, dense W x H
+    uint8_t *pool = nullptr; // kPoolFrames frames, dense W x H
     std::vector<int> free_slots;
     std::deque<RingFrame> ring;
     int income_slot = -1;
@@ -108,7 +108,8 @@ private:
     int frame_index = 0;
     bool initialized = false;
     Outcome outcome = kSkip;
-    bool has_ref = false; // the pool's last slot holds the last result's image
+    int ref_slot = -1;    // slot of the last result's image (none before the first)
+    std::vector<unsigned char> held; // per slot: holders (step, ring, last result)
     int out_parity = 0;   // output buffer of the last result
     SE3f T_world_ref;
     // semi-dense tracker: float images (keyframe / incoming, roles swap on a
@@ -123,7 +124,9 @@ private:
     SE3f sd_T;      // T_income<-key of this frame's step
   };
 
-  Outcome begin_frame(int i, const uint8_t *img, size_t stride, const float *T);
+  Outcome begin_frame(int i, const float *T);
+  void upload(int i, const uint8_t *img, size_t stride);
+  void release(int i, int slot, int parity);
   void end_frame(int i, int parity);
   // one step of the streams in `which` (see submit)
   void step(const std::vector<int> &which, const uint8_t *const *imgs, const size_t *strides,
@@ -137,8 +140,8 @@ private:
   {
     return s.pool + (size_t)slot * s.d.W * s.d.H;
   }
-  uint8_t *ref_ptr(const State &s) const { return frame_ptr(s, QM_RING_CAPACITY + 2); }
-  void keep_reference(State &s);
+  uint8_t *ref_ptr(const State &s) const { return frame_ptr(s, s.ref_slot); }
+  void keep_reference(int i, int parity);
   // enqueues the semi-dense step of the streams in `which` on the engine
   // stream (after their uploads)
   void semidense_step(const std::vector<int> &which, int parity);
@@ -148,11 +151,13 @@ private:
   std::unique_ptr<Engine> eng_;
   std::vector<int> last_active_;
   std::mutex mu_;
-  // pipelining: uploads and downloads run on their own streams; per step
+  // pipelining: uploads and downloads run on their own streams, branch by
+  // branch (ev_in_: a branch's frames are up); per step
   // parity, events mark the end of its uploads, of its pipeline and of its
   // downloads, and the frame slots it freed wait in `pending_` until then
   cudaStream_t up_ = nullptr, down_ = nullptr;
   cudaEvent_t ev_up_[2] = {}, ev_comp_[2] = {}, ev_done_[2] = {};
+  cudaEvent_t ev_in_[kMaxBranches] = {};
   std::vector<std::pair<int, int>> pending_[2]; // (stream, slot)
   bool inflight_[2] = {false, false};
   long step_ = 0;
