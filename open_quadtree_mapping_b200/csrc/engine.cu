@@ -52,14 +52,14 @@ struct Stages
 };
 
 std::vector<int> stage_blocks(const Shape &s, const JobLayout &lay, const qm_params &p,
-                              const Tune &tune)
+                              const Tune &tune, int cost_split)
 {
   const Stages st{p.bp_levels};
   std::vector<int> b(st.count(), 0);
   const int L = p.bp_levels;
   const int D = s.D;
   b[st.qt()] = quadtree_blocks(s.W, s.H, p.qt_max_level);
-  b[st.cost()] = cost_blocks(lay.lw[0], lay.lh[0]);
+  b[st.cost()] = cost_tiles(lay.lw[0], lay.lh[0]) * cost_split;
   // pyramid and message kernels move float4 groups of hypotheses
   for (int l = 1; l < L; ++l)
     b[st.pyr(l)] = cdiv((long)lay.lw[l] * lay.lh[l] * (D / 4), kFlatThreads);
@@ -90,6 +90,7 @@ struct StageTable
   std::vector<int> job_d;          // per job: hypothesis count
   std::vector<long> level_cells;   // per job and BP level: cells
   int max_w = 0, max_h = 0;        // longest lines of the row / column solves
+  int cost_split = 1;              // blocks per tile of the cost kernel
   Tune tune;                       // launch shapes the blocks were counted for
 
   int begin(int stage, int j) const { return hprefix[(size_t)stage * (n + 1) + j]; }
@@ -191,7 +192,7 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
   all(kQuadtree, st.qt(), [&](const Batch &b, int g) { launch_quadtree(b, g, kp, s); });
   const int max_d = T.dvals.empty() ? 0 : T.dvals.back();
   all(kCost, st.cost(),
-      [&](const Batch &b, int g) { launch_cost(b, g, ar, max_d, s, T.tune.cost_blocks); });
+      [&](const Batch &b, int g) { launch_cost(b, g, ar, max_d, T.cost_split, s, T.tune.cost_blocks); });
   for (int l = 1; l < L; ++l)
     all(kPyramid, st.pyr(l), [&](const Batch &b, int g) { launch_pyramid(b, g, l, s); });
   // BP, coarse to fine.  Per hypothesis count the top levels lc[..]..L-1 whose
@@ -203,7 +204,8 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
   auto any_of = [&](int d, int j0, int j1) {
     return std::find(T.job_d.begin() + j0, T.job_d.begin() + j1, d) != T.job_d.begin() + j1;
   };
-  for (size_t di = 0; coarse_cells > 0 && di < T.dvals.size(); ++di)
+  const bool coarse = coarse_cells > 0 && in(st.sweep(L - 1));
+  for (size_t di = 0; coarse && di < T.dvals.size(); ++di)
   {
     const int d = T.dvals[di];
     long cells[kMaxLevels] = {};
@@ -217,7 +219,7 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
       }
     CoarsePlan cp;
     std::memset(&cp, 0, sizeof(cp));
-    if (jobs == 0 || !in(st.sweep(L - 1)) ||
+    if (jobs == 0 ||
         !coarse_plan(cp, d, cells, L, p.bp_iters, coarse_cells, jobs, ar))
       continue;
     lc[di] = cp.lo;
@@ -712,13 +714,17 @@ std::unique_ptr<TableBuf> Engine::build_table(const std::vector<int> &active, co
   std::vector<int> ds;
   StageTable &T = tb->table;
   T.tune = tune;
+  long tiles = 0;
+  for (int j : active)
+    tiles += cost_tiles(layouts_[j].lw[0], layouts_[j].lh[0]);
+  T.cost_split = cost_split(tiles);
   for (int i = 0; i < n; ++i)
   {
     const int j = active[i];
     ds.push_back(shapes_[j].D);
     T.max_w = std::max(T.max_w, shapes_[j].W);
     T.max_h = std::max(T.max_h, shapes_[j].H);
-    per_job.push_back(stage_blocks(shapes_[j], layouts_[j], params_, tune));
+    per_job.push_back(stage_blocks(shapes_[j], layouts_[j], params_, tune, T.cost_split));
     for (int l = 0; l < L; ++l)
       T.level_bytes.push_back((size_t)5 * layouts_[j].lw[l] * layouts_[j].lh[l] * shapes_[j].D *
                               sizeof(float));
@@ -821,7 +827,7 @@ Plan &Engine::plan_for(const std::vector<int> &active)
 static Tune candidate(int c, int max_w, int max_h)
 {
   static const int kWarps[3] = {4, 8, 16}, kRows[3] = {1, 2, 4}, kCols[3] = {2, 4, 8};
-  static const int kCostB[3] = {4, kCostBlocks, 3};
+  static const int kCostB[3] = {5, kCostBlocks, 3};
   Tune t;
   t.sweep_warps = t.extract_warps = kWarps[c];
   t.cost_blocks = kCostB[c];
@@ -1152,7 +1158,8 @@ int run_range(const Batch &B, const Shape &s, const qm_params &p, int first, int
 {
   const JobLayout lay = JobLayout::make(s, p.bp_levels);
   StageTable T;
-  T.add_jobs({stage_blocks(s, lay, p, T.tune)}, {s.D});
+  T.cost_split = cost_split(cost_tiles(lay.lw[0], lay.lh[0]));
+  T.add_jobs({stage_blocks(s, lay, p, T.tune, T.cost_split)}, {s.D});
   T.max_w = s.W;
   T.max_h = s.H;
   for (int l = 0; l < p.bp_levels; ++l)

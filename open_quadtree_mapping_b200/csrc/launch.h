@@ -24,7 +24,7 @@ constexpr int kColLines = 4;
 constexpr int kMaxRowWarps = 4;
 constexpr int kMaxColLines = 8;
 // cost kernel: resident blocks of 256 threads per SM it is compiled for
-constexpr int kCostBlocks = 5;
+constexpr int kCostBlocks = 4;
 // longest lines the solvers' shared memory holds
 constexpr int kMaxRowLen = 4096;
 constexpr int kMaxColLen = 2048;
@@ -54,10 +54,13 @@ void launch_quadtree(const Batch &B, int blocks, KParams kp, cudaStream_t s);
 // cells per block of the cost kernel (one tile of a cell row)
 constexpr int kCostCells = 32;
 constexpr int kMaxHyp = 128;
-int cost_blocks(int cw, int ch);
-// max_d: largest hypothesis count of the batch (sizes the shared tile);
-// blocks_per_sm: 3, 4 or 5, the instance's register budget
-void launch_cost(const Batch &B, int blocks, int arith, int max_d, cudaStream_t s,
+int cost_tiles(int cw, int ch);
+// blocks per tile when the launch's jobs have `tiles` tiles in all
+int cost_split(long tiles);
+// max_d: largest hypothesis count of the batch (sizes the shared tile); split:
+// blocks per tile (1, 2 or 4); blocks_per_sm: 3, 4 or 5, the instance's
+// register budget
+void launch_cost(const Batch &B, int blocks, int arith, int max_d, int split, cudaStream_t s,
                  int blocks_per_sm = kCostBlocks);
 void launch_pyramid(const Batch &B, int blocks, int level, cudaStream_t s);
 // writes the inherited messages of level `level` that its sweeps will read
