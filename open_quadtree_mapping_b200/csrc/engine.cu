@@ -51,15 +51,26 @@ struct Stages
   int count() const { return 6 + 3 * L; }
 };
 
+// How the work of one launch is cut, by the size of all its jobs together.
+struct Cuts
+{
+  int cost_split = 1;                   // blocks per tile of the cost kernel
+  int transform_px = 4, update_px = 8;  // pixels per thread of the fusion kernels
+  static Cuts of(long tiles, long pixels)
+  {
+    return Cuts{qm::cost_split(tiles), fuse_transform_px(pixels), fuse_px(pixels)};
+  }
+};
+
 std::vector<int> stage_blocks(const Shape &s, const JobLayout &lay, const qm_params &p,
-                              const Tune &tune, int cost_split)
+                              const Tune &tune, const Cuts &cuts)
 {
   const Stages st{p.bp_levels};
   std::vector<int> b(st.count(), 0);
   const int L = p.bp_levels;
   const int D = s.D;
   b[st.qt()] = quadtree_blocks(s.W, s.H, p.qt_max_level);
-  b[st.cost()] = cost_tiles(lay.lw[0], lay.lh[0]) * cost_split;
+  b[st.cost()] = cost_tiles(lay.lw[0], lay.lh[0]) * cuts.cost_split;
   // pyramid and message kernels move float4 groups of hypotheses
   for (int l = 1; l < L; ++l)
     b[st.pyr(l)] = cdiv((long)lay.lw[l] * lay.lh[l] * (D / 4), kFlatThreads);
@@ -73,8 +84,8 @@ std::vector<int> stage_blocks(const Shape &s, const JobLayout &lay, const qm_par
   b[st.extract()] = cdiv((long)lay.lw[0] * lay.lh[0], epb);
   b[st.row()] = cdiv(s.H, tune.row_warps);
   b[st.col()] = cdiv(s.W, tune.col_lines);
-  b[st.ftrans()] = cdiv((long)s.W * s.H, kFlatThreads * kFuseTransformPx);
-  b[st.fupd()] = cdiv((long)s.W * s.H, kFlatThreads * kFuseUpdatePx);
+  b[st.ftrans()] = cdiv((long)s.W * s.H, kFlatThreads * cuts.transform_px);
+  b[st.fupd()] = cdiv((long)s.W * s.H, kFlatThreads * cuts.update_px);
   return b;
 }
 
@@ -90,7 +101,7 @@ struct StageTable
   std::vector<int> job_d;          // per job: hypothesis count
   std::vector<long> level_cells;   // per job and BP level: cells
   int max_w = 0, max_h = 0;        // longest lines of the row / column solves
-  int cost_split = 1;              // blocks per tile of the cost kernel
+  Cuts cuts;                       // how the launch's work is cut
   Tune tune;                       // launch shapes the blocks were counted for
 
   int begin(int stage, int j) const { return hprefix[(size_t)stage * (n + 1) + j]; }
@@ -192,7 +203,7 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
   all(kQuadtree, st.qt(), [&](const Batch &b, int g) { launch_quadtree(b, g, kp, s); });
   const int max_d = T.dvals.empty() ? 0 : T.dvals.back();
   all(kCost, st.cost(),
-      [&](const Batch &b, int g) { launch_cost(b, g, ar, max_d, T.cost_split, s, T.tune.cost_blocks); });
+      [&](const Batch &b, int g) { launch_cost(b, g, ar, max_d, T.cuts.cost_split, s, T.tune.cost_blocks); });
   for (int l = 1; l < L; ++l)
     all(kPyramid, st.pyr(l), [&](const Batch &b, int g) { launch_pyramid(b, g, l, s); });
   // BP, coarse to fine.  Per hypothesis count the top levels lc[..]..L-1 whose
@@ -283,8 +294,8 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
     launch_col_solve(b, g, kp, ar, T.max_h, s, T.tune.col_lines);
   });
   all(kFuseTransform, st.ftrans(),
-      [&](const Batch &b, int g) { launch_fuse_transform(b, g, ar, s); });
-  all(kFuseUpdate, st.fupd(), [&](const Batch &b, int g) { launch_fuse_update(b, g, s); });
+      [&](const Batch &b, int g) { launch_fuse_transform(b, g, T.cuts.transform_px, ar, s); });
+  all(kFuseUpdate, st.fupd(), [&](const Batch &b, int g) { launch_fuse_update(b, g, T.cuts.update_px, s); });
   check(cudaGetLastError(), "kernel launch");
   return n;
 }
@@ -714,17 +725,20 @@ std::unique_ptr<TableBuf> Engine::build_table(const std::vector<int> &active, co
   std::vector<int> ds;
   StageTable &T = tb->table;
   T.tune = tune;
-  long tiles = 0;
+  long tiles = 0, pixels = 0;
   for (int j : active)
+  {
     tiles += cost_tiles(layouts_[j].lw[0], layouts_[j].lh[0]);
-  T.cost_split = cost_split(tiles);
+    pixels += (long)shapes_[j].W * shapes_[j].H;
+  }
+  T.cuts = Cuts::of(tiles, pixels);
   for (int i = 0; i < n; ++i)
   {
     const int j = active[i];
     ds.push_back(shapes_[j].D);
     T.max_w = std::max(T.max_w, shapes_[j].W);
     T.max_h = std::max(T.max_h, shapes_[j].H);
-    per_job.push_back(stage_blocks(shapes_[j], layouts_[j], params_, tune, T.cost_split));
+    per_job.push_back(stage_blocks(shapes_[j], layouts_[j], params_, tune, T.cuts));
     for (int l = 0; l < L; ++l)
       T.level_bytes.push_back((size_t)5 * layouts_[j].lw[l] * layouts_[j].lh[l] * shapes_[j].D *
                               sizeof(float));
@@ -1158,8 +1172,8 @@ int run_range(const Batch &B, const Shape &s, const qm_params &p, int first, int
 {
   const JobLayout lay = JobLayout::make(s, p.bp_levels);
   StageTable T;
-  T.cost_split = cost_split(cost_tiles(lay.lw[0], lay.lh[0]));
-  T.add_jobs({stage_blocks(s, lay, p, T.tune, T.cost_split)}, {s.D});
+  T.cuts = Cuts::of(cost_tiles(lay.lw[0], lay.lh[0]), (long)s.W * s.H);
+  T.add_jobs({stage_blocks(s, lay, p, T.tune, T.cuts)}, {s.D});
   T.max_w = s.W;
   T.max_h = s.H;
   for (int l = 0; l < p.bp_levels; ++l)

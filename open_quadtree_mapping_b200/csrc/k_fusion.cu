@@ -120,26 +120,26 @@ __device__ __forceinline__ void transform_px(const JobDesc &J, int idx, float4 i
   }
 }
 
-// kFuseTransformPx pixels per thread, their seeds loaded before any is
-// processed (the loads are the latency that bounds this pass)
-template <class A>
+// PX pixels per thread, their seeds loaded before any is processed (the loads
+// are the latency that bounds this pass)
+template <class A, int PX>
 __global__ void __launch_bounds__(kFlatThreads)
     k_fuse_transform(const __grid_constant__ Batch B)
 {
   int lb;
   const JobDesc &J = job_of(B, lb);
   const int npx = J.W * J.H;
-  const int base = lb * (int)blockDim.x * kFuseTransformPx + (int)threadIdx.x;
+  const int base = lb * (int)blockDim.x * PX + (int)threadIdx.x;
   const float inv_w = 1.0f / (float)J.W;
-  float4 info[kFuseTransformPx];
+  float4 info[PX];
 #pragma unroll
-  for (int u = 0; u < kFuseTransformPx; ++u)
+  for (int u = 0; u < PX; ++u)
   {
     const int idx = base + u * (int)blockDim.x;
     info[u] = idx < npx ? J.seeds_in[idx] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
 #pragma unroll
-  for (int u = 0; u < kFuseTransformPx; ++u)
+  for (int u = 0; u < PX; ++u)
   {
     const int idx = base + u * (int)blockDim.x;
     if (idx < npx)
@@ -243,8 +243,8 @@ __device__ __forceinline__ void update_px(const JobDesc &J, int idx, double dep,
   J.seeds_out[idx] = make_float4((float)a_p, (float)b_p, (float)mu_p, (float)s2_p);
 }
 
-// A block owns kFlatThreads * kFuseUpdatePx consecutive pixels and walks
-// them in kFuseUpdatePx steps of one pixel per thread.  The pixel chain
+// A block owns kFlatThreads * px consecutive pixels and walks them in px steps
+// of one pixel per thread.  The pixel chain
 // (key -> source, for an empty pixel through its neighbours' keys -> source
 // seed -> FP64 update) is software-pipelined: while step j's update runs,
 // step j+1's source seed and step j+2's key and depth are already in flight,
@@ -252,13 +252,13 @@ __device__ __forceinline__ void update_px(const JobDesc &J, int idx, double dep,
 // Every pixel's result depends only on its own inputs and on keys this
 // kernel does not write, so the order changes nothing.
 __global__ void __launch_bounds__(kFlatThreads)
-    k_fuse_update(const __grid_constant__ Batch B)
+    k_fuse_update(const __grid_constant__ Batch B, int px)
 {
   int lb;
   const JobDesc &J = job_of(B, lb);
   const int npx = J.W * J.H;
   const int step = (int)blockDim.x;
-  const int base = lb * step * kFuseUpdatePx + (int)threadIdx.x;
+  const int base = lb * step * px + (int)threadIdx.x;
   const float inv_w = 1.0f / (float)J.W;
   auto pix = [&](int j) { return base + j * step; };
   // step j: depth and key (loaded two steps ahead), source and its seed
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kFlatThreads)
       dep0 = J.dense[i0];
       key0 = J.zkey[i0];
     }
-    if (kFuseUpdatePx > 1 && i1 < npx)
+    if (px > 1 && i1 < npx)
     {
       dep1 = J.dense[i1];
       key1 = J.zkey[i1];
@@ -284,14 +284,14 @@ __global__ void __launch_bounds__(kFlatThreads)
     if (pre0 > 0)
       src0 = J.seeds_in[pre0];
   }
-  for (int j = 0; j < kFuseUpdatePx; ++j)
+  for (int j = 0; j < px; ++j)
   {
     const int i0 = pix(j), i1 = pix(j + 1), i2 = pix(j + 2);
     if (i0 >= npx)
       break; // later steps are further out
     int pre1 = 0;
     float4 src1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (j + 1 < kFuseUpdatePx && i1 < npx)
+    if (j + 1 < px && i1 < npx)
     {
       pre1 = resolve_source(J, i1, key1, inv_w);
       if (pre1 > 0)
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(kFlatThreads)
     }
     float dep2 = 0.0f;
     unsigned long long key2 = kEmpty;
-    if (j + 2 < kFuseUpdatePx && i2 < npx)
+    if (j + 2 < px && i2 < npx)
     {
       dep2 = J.dense[i2];
       key2 = J.zkey[i2];
@@ -331,17 +331,27 @@ void launch_seed_variance(const float4 *seeds, float *out, long n, cudaStream_t 
         seeds, out, n);
 }
 
-void launch_fuse_transform(const Batch &B, int blocks, int arith, cudaStream_t s)
+// The pipelined walk pays when there are blocks for every SM several times
+// over; below that a thread with eight pixels is only a longer chain.  Update /
+// transform of one image, 8 and 4 pixels per thread before: 160x128 11.1 / 4.2
+// -> 3.6 / 2.9 us, 752x480 14.7 / 5.6 -> 10.1 / 5.3, 1280x720 23.0 / 10.1 -> 19.5
+// / 9.3; at 1920x1080 8 pixels 38.5, 2 pixels 40.2 (transform 18.6 and 17.6).
+int fuse_px(long pixels) { return pixels <= 160000 ? 1 : pixels <= 1200000 ? 2 : 8; }
+int fuse_transform_px(long pixels) { return pixels <= 2100000 ? 1 : 4; }
+
+void launch_fuse_transform(const Batch &B, int blocks, int px, int arith, cudaStream_t s)
 {
   if (arith == QM_ARITH_IEEE)
-    k_fuse_transform<ArithIeee><<<blocks, kFlatThreads, 0, s>>>(B);
+    px > 1 ? k_fuse_transform<ArithIeee, 4><<<blocks, kFlatThreads, 0, s>>>(B)
+           : k_fuse_transform<ArithIeee, 1><<<blocks, kFlatThreads, 0, s>>>(B);
   else
-    k_fuse_transform<ArithRef><<<blocks, kFlatThreads, 0, s>>>(B);
+    px > 1 ? k_fuse_transform<ArithRef, 4><<<blocks, kFlatThreads, 0, s>>>(B)
+           : k_fuse_transform<ArithRef, 1><<<blocks, kFlatThreads, 0, s>>>(B);
 }
 
-void launch_fuse_update(const Batch &B, int blocks, cudaStream_t s)
+void launch_fuse_update(const Batch &B, int blocks, int px, cudaStream_t s)
 {
-  k_fuse_update<<<blocks, kFlatThreads, 0, s>>>(B);
+  k_fuse_update<<<blocks, kFlatThreads, 0, s>>>(B, px);
 }
 
 } // namespace qm

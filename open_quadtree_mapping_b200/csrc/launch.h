@@ -129,14 +129,14 @@ void launch_row_solve(const Batch &B, int blocks, KParams kp, int arith, int max
                       cudaStream_t s, int rows = kRowWarps);
 void launch_col_solve(const Batch &B, int blocks, KParams kp, int arith, int max_h,
                       cudaStream_t s, int lines = kColLines);
-// pixels per thread of the fusion transform and update (their blocks cover
-// kFlatThreads times as many; the update walks its pixels as a pipeline)
-constexpr int kFuseTransformPx = 4;
-constexpr int kFuseUpdatePx = 8;
-void launch_fuse_transform(const Batch &B, int blocks, int arith, cudaStream_t s);
+// Pixels per thread of the fusion update (it walks them as a pipeline) and of
+// the transform (1 or 4) when the launch's jobs have `pixels` pixels in all
+int fuse_px(long pixels);
+int fuse_transform_px(long pixels);
+void launch_fuse_transform(const Batch &B, int blocks, int px, int arith, cudaStream_t s);
 // hole filling + posterior update (reads the z-buffer keys, leaves them set:
 // the next frame's row solve resets them)
-void launch_fuse_update(const Batch &B, int blocks, cudaStream_t s);
+void launch_fuse_update(const Batch &B, int blocks, int px, cudaStream_t s);
 // out[i] = seeds[i].w (the fused variance sigma^2), n pixels
 void launch_seed_variance(const float4 *seeds, float *out, long n, cudaStream_t s);
 
