@@ -983,6 +983,7 @@ Batch Engine::upload(int n, cudaStream_t s)
   std::memset(&B, 0, sizeof(B));
   B.jobs = d_block_.run;
   B.njobs = n;
+  B.early = n == 1 ? 1 : 0; // one stream: nothing else fills the GPU
   B.slot_ptr = d_block_.slot_ptr;
   B.slot_T = d_block_.slot_T;
   B.slot_w = d_block_.slot_w;
@@ -1163,6 +1164,7 @@ Batch single(const JobDesc &J)
   std::memset(&B, 0, sizeof(B));
   B.jobs = nullptr;
   B.njobs = 1;
+  B.early = 1;
   B.one = J;
   return B;
 }

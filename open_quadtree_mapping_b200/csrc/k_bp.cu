@@ -115,6 +115,7 @@ __device__ __forceinline__ float mean_of(float sum)
 __global__ void __launch_bounds__(kFlatThreads)
     k_pyramid(const __grid_constant__ Batch B, int level)
 {
+  after_previous();
   int lb;
   const JobDesc &J = job_of(B, lb);
   const LevelDesc &Lf = J.lv[level - 1];
@@ -170,6 +171,7 @@ __device__ __forceinline__ bool bp_skipped(const JobDesc &J, int level, int x, i
 __global__ void __launch_bounds__(kFlatThreads)
     k_msg_inherit(const __grid_constant__ Batch B, int level, int iters, int qt_max)
 {
+  after_previous();
   int lb;
   const JobDesc &J = job_of(B, lb);
   const LevelDesc &F = J.lv[level];
@@ -466,6 +468,7 @@ __global__ void __launch_bounds__(kMaxCellWarps * 32, 4)
     k_bp_sweep(const __grid_constant__ Batch B, int level, int parity, int first, int inherit,
                KParams kp)
 {
+  after_previous();
   constexpr int G = HypLayout<D>::G;
   int lb;
   const JobDesc &J = job_of(B, lb);
@@ -487,6 +490,7 @@ __global__ void __launch_bounds__(kMaxCellWarps * 32, 4)
     k_bp_sweep_io(const __grid_constant__ Batch B, int level, int parity, int first,
                   const __grid_constant__ SweepIO io, KParams kp)
 {
+  after_previous();
   constexpr int G = HypLayout<D>::G;
   const LevelDesc &L = B.one.lv[level];
   const int item0 = ((int)blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5)) * G;
@@ -585,6 +589,7 @@ __global__ void __launch_bounds__(kCoarseMaxThreads, 1)
     k_bp_coarse(const __grid_constant__ Batch B, int j0, const __grid_constant__ CoarsePlan plan,
                 KParams kp)
 {
+  after_previous();
   using QL = QuadLayout<D>;
   constexpr int LPC = QL::LPC, G = 32 / LPC;
   const int threads = blockDim.x, groups = threads / LPC;
@@ -767,6 +772,7 @@ template <int D, int ARITH>
 __global__ void __launch_bounds__(kMaxCellWarps * 32)
     k_extract(const __grid_constant__ Batch B)
 {
+  after_previous();
   using HL = HypLayout<D>;
   constexpr int NV = HL::NV, LPC = HL::LPC, G = HL::G;
   int lb;
@@ -873,11 +879,9 @@ void sweep_d(const Batch &B, int blocks, int level, int parity, int first, int i
              KParams kp, int arith, int warps, cudaStream_t s)
 {
   if (arith == QM_ARITH_IEEE)
-    k_bp_sweep<D, QM_ARITH_IEEE>
-        <<<blocks, warps * 32, 0, s>>>(B, level, parity, first, inherit, kp);
+    launch_kernel(k_bp_sweep<D, QM_ARITH_IEEE>, blocks, warps * 32, 0, s, B.early, B, level, parity, first, inherit, kp);
   else
-    k_bp_sweep<D, QM_ARITH_REFERENCE>
-        <<<blocks, warps * 32, 0, s>>>(B, level, parity, first, inherit, kp);
+    launch_kernel(k_bp_sweep<D, QM_ARITH_REFERENCE>, blocks, warps * 32, 0, s, B.early, B, level, parity, first, inherit, kp);
 }
 
 // Opt-ins of one k_bp_coarse instance on the current device (large shared
@@ -920,7 +924,9 @@ void coarse_k(const Batch &B, int j0, int jobs, const CoarsePlan &plan, KParams 
 {
   coarse_prepare<D, ARITH, HIST>(plan.ctas);
   cudaLaunchConfig_t c = {};
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = plan.ctas;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
@@ -929,7 +935,7 @@ void coarse_k(const Batch &B, int j0, int jobs, const CoarsePlan &plan, KParams 
   c.dynamicSmemBytes = coarse_smem<D>(plan.per, plan.data_smem != 0);
   c.stream = s;
   c.attrs = at;
-  c.numAttrs = 1;
+  c.numAttrs = B.early ? 2 : 1;
   cudaLaunchKernelEx(&c, k_bp_coarse<D, ARITH, HIST>, B, j0, plan, kp);
 }
 
@@ -975,20 +981,18 @@ void sweep_io_d(const Batch &B, int blocks, int level, int it, const SweepIO &io
                 int arith, cudaStream_t s)
 {
   if (arith == QM_ARITH_IEEE)
-    k_bp_sweep_io<D, QM_ARITH_IEEE>
-        <<<blocks, kCellWarps * 32, 0, s>>>(B, level, it & 1, it == 0, io, kp);
+    launch_kernel(k_bp_sweep_io<D, QM_ARITH_IEEE>, blocks, kCellWarps * 32, 0, s, B.early, B, level, it & 1, it == 0, io, kp);
   else
-    k_bp_sweep_io<D, QM_ARITH_REFERENCE>
-        <<<blocks, kCellWarps * 32, 0, s>>>(B, level, it & 1, it == 0, io, kp);
+    launch_kernel(k_bp_sweep_io<D, QM_ARITH_REFERENCE>, blocks, kCellWarps * 32, 0, s, B.early, B, level, it & 1, it == 0, io, kp);
 }
 
 template <int D>
 void extract_d(const Batch &B, int blocks, int arith, int warps, cudaStream_t s)
 {
   if (arith == QM_ARITH_IEEE)
-    k_extract<D, QM_ARITH_IEEE><<<blocks, warps * 32, 0, s>>>(B);
+    launch_kernel(k_extract<D, QM_ARITH_IEEE>, blocks, warps * 32, 0, s, B.early, B);
   else
-    k_extract<D, QM_ARITH_REFERENCE><<<blocks, warps * 32, 0, s>>>(B);
+    launch_kernel(k_extract<D, QM_ARITH_REFERENCE>, blocks, warps * 32, 0, s, B.early, B);
 }
 
 } // namespace
@@ -1029,13 +1033,13 @@ int bp_cells_per_warp(int d)
 void launch_pyramid(const Batch &B, int blocks, int level,
                     cudaStream_t s)
 {
-  k_pyramid<<<blocks, kFlatThreads, 0, s>>>(B, level);
+  launch_kernel(k_pyramid, blocks, kFlatThreads, 0, s, B.early, B, level);
 }
 
 void launch_msg_inherit(const Batch &B, int blocks, int level, int iters, int qt_max,
                         cudaStream_t s)
 {
-  k_msg_inherit<<<blocks, kFlatThreads, 0, s>>>(B, level, iters, qt_max);
+  launch_kernel(k_msg_inherit, blocks, kFlatThreads, 0, s, B.early, B, level, iters, qt_max);
 }
 
 // A batch with mixed hypothesis counts launches one sweep per count present;

@@ -163,6 +163,7 @@ template <class A, int MINB, bool WORDS>
 __global__ void __launch_bounds__(kFlatThreads, MINB)
     k_cost(const __grid_constant__ Batch B, int split)
 {
+  after_previous();
   // sum of absolute differences (low 20 bits: at most 32 slots * 9 * 255) and
   // number of valid slots of the tile, [kCostCells][D + 1] (the padding keeps
   // lanes that add to one hypothesis of different cells on different banks)
@@ -452,9 +453,9 @@ template <int MINB, bool WORDS>
 void cost_minb(const Batch &B, int blocks, int arith, int split, size_t sm, cudaStream_t s)
 {
   if (arith == QM_ARITH_IEEE)
-    k_cost<ArithIeee, MINB, WORDS><<<blocks, kFlatThreads, sm, s>>>(B, split);
+    launch_kernel(k_cost<ArithIeee, MINB, WORDS>, blocks, kFlatThreads, sm, s, B.early, B, split);
   else
-    k_cost<ArithRef, MINB, WORDS><<<blocks, kFlatThreads, sm, s>>>(B, split);
+    launch_kernel(k_cost<ArithRef, MINB, WORDS>, blocks, kFlatThreads, sm, s, B.early, B, split);
 }
 
 // Slot images whose rows all start on a word: always in the engine's frame

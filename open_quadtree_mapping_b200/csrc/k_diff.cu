@@ -119,6 +119,7 @@ template <int D, class R>
 __global__ void __launch_bounds__(kDiffWarps * 32)
     k_soft_readout(const DiffBpR<R> a, int backward)
 {
+  after_previous();
   using M = Real<R>;
   constexpr int NV = (D + 31) / 32;
   const int cell = blockIdx.x * kDiffWarps + (threadIdx.x >> 5);
@@ -410,6 +411,7 @@ __device__ __forceinline__ void bwd_cell(const DiffBpR<R> &a, int x, int y, int 
 template <int D, class R>
 __global__ void __launch_bounds__(kDiffWarps * 32) k_bp_sweep_bwd(const DiffBpR<R> a)
 {
+  after_previous();
   using M = Real<R>;
   constexpr int NV = (D + 31) / 32;
   __shared__ double s_gp[2][kDiffWarps];
@@ -445,6 +447,7 @@ template <class R>
 __global__ void __launch_bounds__(256)
     k_msg_downsample(const DiffBpR<R> a, const MsgPtrsR<R> parent, int pw, int ph)
 {
+  after_previous();
   const int D = a.D;
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long)pw * ph * D)
@@ -860,6 +863,7 @@ template <bool BWD>
 __global__ void __launch_bounds__(64) k_upw_rows(const DiffUp u)
 {
   const double *tab = upw_table(u.sigma);
+  after_previous();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int y = blockIdx.x * (int)(blockDim.x >> 5) + warp, n = u.W;
   if (y >= u.H)
@@ -914,6 +918,7 @@ template <bool BWD>
 __global__ void __launch_bounds__(128) k_upw_cols(const DiffUp u)
 {
   const double *tab = upw_table(u.sigma);
+  after_previous();
   const int C = blockDim.x >> 5, n = u.H;
   const int kt = (int)threadIdx.x / C, ct = (int)threadIdx.x - kt * C;
   const int xt = blockIdx.x * C + ct;
@@ -1093,6 +1098,7 @@ __device__ __forceinline__ Dual dsqrt(Dual a)
 // prior of the pixel (table and transformed seeds of the forward fusion)
 __global__ void __launch_bounds__(256) k_fuse_bwd(DiffFuse f)
 {
+  after_previous();
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long)f.W * f.H)
     return;
@@ -1136,15 +1142,14 @@ template <int D, class R>
 void readout_d(const DiffBpR<R> &a, int backward, cudaStream_t s)
 {
   const int cells = a.w * a.h;
-  k_soft_readout<D, R><<<(cells + kDiffWarps - 1) / kDiffWarps, kDiffWarps * 32, 0, s>>>(
-      a, backward);
+  launch_kernel(k_soft_readout<D, R>, (cells + kDiffWarps - 1) / kDiffWarps, kDiffWarps * 32, 0, s, 1, a, backward);
 }
 
 template <int D, class R>
 void bwd_d(const DiffBpR<R> &a, cudaStream_t s)
 {
   const int items = ((a.w + 1) / 2) * a.h;
-  k_bp_sweep_bwd<D, R><<<(items + kDiffWarps - 1) / kDiffWarps, kDiffWarps * 32, 0, s>>>(a);
+  launch_kernel(k_bp_sweep_bwd<D, R>, (items + kDiffWarps - 1) / kDiffWarps, kDiffWarps * 32, 0, s, 1, a);
 }
 
 template <class F>
@@ -1190,7 +1195,7 @@ void downsample(const DiffBpR<R> &a, const MsgPtrsR<R> &parent, int pw, int ph, 
 {
   const long n = (long)pw * ph * a.D;
   if (n > 0)
-    k_msg_downsample<R><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, parent, pw, ph);
+    launch_kernel(k_msg_downsample<R>, (unsigned)((n + 255) / 256), 256, 0, s, 1, a, parent, pw, ph);
 }
 } // namespace
 
@@ -1273,8 +1278,7 @@ void upw_rows(const DiffUp &u, cudaStream_t s)
 {
   const int c = upw_lines(u.W, 2);
   if (c > 0)
-    k_upw_rows<BWD><<<(u.H + c - 1) / c, 32 * c,
-                      kUpwTableBytes + c * upw_line_doubles(u.W) * sizeof(double), s>>>(u);
+    launch_kernel(k_upw_rows<BWD>, (u.H + c - 1) / c, 32 * c, kUpwTableBytes + c * upw_line_doubles(u.W) * sizeof(double), s, 1, u);
   else if (BWD)
     k_upw_rows_bwd<<<(u.H + 63) / 64, 64, 0, s>>>(u);
   else
@@ -1286,8 +1290,7 @@ void upw_cols(const DiffUp &u, cudaStream_t s)
 {
   const int c = upw_lines(u.H, 4);
   if (c > 0)
-    k_upw_cols<BWD><<<(u.W + c - 1) / c, 32 * c,
-                      kUpwTableBytes + c * upw_line_doubles(u.H) * sizeof(double), s>>>(u);
+    launch_kernel(k_upw_cols<BWD>, (u.W + c - 1) / c, 32 * c, kUpwTableBytes + c * upw_line_doubles(u.H) * sizeof(double), s, 1, u);
   else if (BWD)
     k_upw_cols_bwd<<<(u.W + 63) / 64, 64, 0, s>>>(u);
   else
@@ -1313,7 +1316,7 @@ void launch_fuse_bwd(const DiffFuse &f, cudaStream_t s)
 {
   const long n = (long)f.W * f.H;
   if (n > 0)
-    k_fuse_bwd<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(f);
+    launch_kernel(k_fuse_bwd, (unsigned)((n + 255) / 256), 256, 0, s, 1, f);
 }
 
 } // namespace qm

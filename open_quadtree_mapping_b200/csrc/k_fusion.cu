@@ -126,6 +126,7 @@ template <class A, int PX>
 __global__ void __launch_bounds__(kFlatThreads)
     k_fuse_transform(const __grid_constant__ Batch B)
 {
+  after_previous();
   int lb;
   const JobDesc &J = job_of(B, lb);
   const int npx = J.W * J.H;
@@ -254,6 +255,7 @@ __device__ __forceinline__ void update_px(const JobDesc &J, int idx, double dep,
 __global__ void __launch_bounds__(kFlatThreads)
     k_fuse_update(const __grid_constant__ Batch B, int px)
 {
+  after_previous();
   int lb;
   const JobDesc &J = job_of(B, lb);
   const int npx = J.W * J.H;
@@ -342,16 +344,16 @@ int fuse_transform_px(long pixels) { return pixels <= 2100000 ? 1 : 4; }
 void launch_fuse_transform(const Batch &B, int blocks, int px, int arith, cudaStream_t s)
 {
   if (arith == QM_ARITH_IEEE)
-    px > 1 ? k_fuse_transform<ArithIeee, 4><<<blocks, kFlatThreads, 0, s>>>(B)
-           : k_fuse_transform<ArithIeee, 1><<<blocks, kFlatThreads, 0, s>>>(B);
+    px > 1 ? launch_kernel(k_fuse_transform<ArithIeee, 4>, blocks, kFlatThreads, 0, s, B.early, B)
+           : launch_kernel(k_fuse_transform<ArithIeee, 1>, blocks, kFlatThreads, 0, s, B.early, B);
   else
-    px > 1 ? k_fuse_transform<ArithRef, 4><<<blocks, kFlatThreads, 0, s>>>(B)
-           : k_fuse_transform<ArithRef, 1><<<blocks, kFlatThreads, 0, s>>>(B);
+    px > 1 ? launch_kernel(k_fuse_transform<ArithRef, 4>, blocks, kFlatThreads, 0, s, B.early, B)
+           : launch_kernel(k_fuse_transform<ArithRef, 1>, blocks, kFlatThreads, 0, s, B.early, B);
 }
 
 void launch_fuse_update(const Batch &B, int blocks, int px, cudaStream_t s)
 {
-  k_fuse_update<<<blocks, kFlatThreads, 0, s>>>(B, px);
+  launch_kernel(k_fuse_update, blocks, kFlatThreads, 0, s, B.early, B, px);
 }
 
 } // namespace qm

@@ -25,6 +25,7 @@ constexpr int kMaxTile = 8; // qt_max <= 3
 __global__ void __launch_bounds__(256)
     k_quadtree(const __grid_constant__ Batch B, KParams kp)
 {
+  after_previous();
   int tile;
   const JobDesc &J = job_of(B, tile);
   const int T = 1 << kp.qt_max;
@@ -158,6 +159,7 @@ template <bool FIVE>
 __global__ void __launch_bounds__(kQtWarps * 32)
     k_quadtree16(const __grid_constant__ Batch B, KParams kp)
 {
+  after_previous();
   __shared__ Node s_quad[kQtWarps];
   int lb;
   const JobDesc &J = job_of(B, lb);
@@ -296,11 +298,11 @@ int quadtree_blocks(int W, int H, int qt_max)
 void launch_quadtree(const Batch &B, int blocks, KParams kp, cudaStream_t s)
 {
   if (kp.qt_max == 4)
-    k_quadtree16<false><<<blocks, kQtWarps * 32, 0, s>>>(B, kp);
+    launch_kernel(k_quadtree16<false>, blocks, kQtWarps * 32, 0, s, B.early, B, kp);
   else if (kp.qt_max == 5)
-    k_quadtree16<true><<<blocks, kQtWarps * 32, 0, s>>>(B, kp);
+    launch_kernel(k_quadtree16<true>, blocks, kQtWarps * 32, 0, s, B.early, B, kp);
   else
-    k_quadtree<<<blocks, 256, 0, s>>>(B, kp);
+    launch_kernel(k_quadtree, blocks, 256, 0, s, B.early, B, kp);
 }
 
 } // namespace qm

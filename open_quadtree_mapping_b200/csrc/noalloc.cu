@@ -162,6 +162,7 @@ extern "C" int qm_upsample_noalloc(const float *sparse, const uint8_t *img, size
     Batch B;
     std::memset(&B, 0, sizeof(B));
     B.njobs = 1;
+    B.early = 1;
     JobDesc &J = B.one;
     J.W = width;
     J.H = height;

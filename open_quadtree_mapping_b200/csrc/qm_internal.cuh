@@ -98,12 +98,23 @@ struct Batch
   int block0;  // global block index of this launch's first block (job groups)
   int uniform; // > 0: every job has this many blocks (job = block / uniform)
   int rev;     // 1: blocks take their work in reverse order (last block first)
+  int early;   // host: 1 = kernels may be launched before their predecessor ends
   const uint8_t *const *slot_ptr; // per slot, device image (null: `slots`)
   const float *slot_T;            // per slot, 12 floats T_slot<-ref
   const int *slot_w;              // per slot, multiplicity
   JobDesc one;
   SlotInline slots;
 };
+
+// First statement of a kernel that touches memory other kernels of the stream
+// write or read: waits until the kernel before it has ended (launched early, see
+// launch_kernel; otherwise there is nothing to wait for), then lets the next one
+// be launched, whose blocks wait here in turn.
+__device__ __forceinline__ void after_previous()
+{
+  asm volatile("griddepcontrol.wait;\n"
+               "griddepcontrol.launch_dependents;\n" ::: "memory");
+}
 
 // Parameters shared by all jobs of a batch (kernel arguments by value).
 struct KParams
