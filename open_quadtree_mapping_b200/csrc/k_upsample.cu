@@ -50,7 +50,7 @@ namespace
 // the 256-entry weight table, then one line after the other.
 extern __shared__ __align__(16) unsigned char g_smem[];
 
-constexpr int kTableBytes = 256 * sizeof(float);
+constexpr int kTableBytes = 256 * sizeof(double);
 
 __device__ __forceinline__ float *smf(int byte_off)
 {
@@ -76,6 +76,15 @@ __host__ __device__ __forceinline__ int line_bytes(int n)
   return 3 * farray_bytes(n) + 32 * seg_pitch(n);
 }
 
+// Distance of the lines of a column stripe: a warp loads and stores 32 / lines
+// consecutive samples of every line, whose banks follow one another when the
+// lines start 128 / lines bytes apart modulo the 128 bytes of a bank row
+// (otherwise all lines start on one bank).
+__host__ __device__ __forceinline__ int stripe_pitch(int n, int lines)
+{
+  return (line_bytes(n) + 127) / 128 * 128 + 128 / lines;
+}
+
 // One line of n samples in shared memory, as byte offsets: rd / ri hold the
 // two right-hand sides (the sparse depth and its indicator), later their
 // forward values and the solution; cp the reciprocal pivots, later the
@@ -87,7 +96,7 @@ struct Line
   int rd, ri, cp, img;
   int n, m, mp;
   unsigned m_inv; // ceil(2^32 / m): k / m = umulhi(k, m_inv) for 0 <= k < 2^20
-  float w_close;  // weight between samples n - 1 and n (the closing weight)
+  double w_close; // lambda * weight between samples n - 1 and n (the closing weight)
   __device__ __forceinline__ int pos(int k) const
   {
     // with m_inv = (2^32 + e) / m, 0 <= e < m, umulhi gives floor(k/m + k e /
@@ -97,7 +106,7 @@ struct Line
   }
 };
 
-__device__ __forceinline__ Line line_at(int base, int n, float w_close)
+__device__ __forceinline__ Line line_at(int base, int n, double w_close)
 {
   Line L;
   const int fb = farray_bytes(n);
@@ -147,19 +156,20 @@ __device__ __forceinline__ float edge_weight(float a, float b, double sigma)
 }
 
 // The weight depends only on |I_k - I_{k-1}| (integers 0..255): a block
-// tabulates edge_weight for every difference once and the passes look it
-// up (the same values the expression gives pixel by pixel).
+// tabulates lambda times edge_weight for every difference once, in the FP64
+// the recurrences need, and the passes look it up.
 template <class A>
-__device__ __forceinline__ void build_weight_table(double sigma)
+__device__ __forceinline__ void build_weight_table(double sigma, double lam)
 {
+  double *tab = reinterpret_cast<double *>(g_smem);
   for (int t = threadIdx.x; t < 256; t += blockDim.x)
-    smf(0)[t] = edge_weight<A>((float)t, 0.0f, sigma);
+    tab[t] = lam * (double)edge_weight<A>((float)t, 0.0f, sigma);
 }
 
-// weight between samples with intensities a and b
-__device__ __forceinline__ float table_weight(int a, int b)
+// lambda * weight between samples with intensities a and b
+__device__ __forceinline__ double table_weight(int a, int b)
 {
-  return smf(0)[a > b ? a - b : b - a];
+  return reinterpret_cast<const double *>(g_smem)[__usad(a, b, 0)];
 }
 
 struct Mat2
@@ -210,8 +220,8 @@ struct Aff
 };
 
 // Walks the lane's segment [s, e) chunk by chunk (s = lane * m, element s at
-// position base = lane * mp): calls f(k, wl[4], wr[4]) with the weights left
-// and right of samples k .. k + 3.  w_0 = 0, w_n = the closing weight, every
+// position base = lane * mp): calls f(k, wl[4], wr[4]) with lambda times the
+// weights left and right of samples k .. k + 3.  w_0 = 0, w_n = the closing weight, every
 // other from the table.  The image bytes of the next chunk are fetched
 // before the current chunk is processed.  A segment that does not end the
 // line holds all m samples, so the sample after it is the next lane's first
@@ -224,15 +234,15 @@ __device__ __forceinline__ void walk_chunks(const Line &L, int s, int e, int bas
     return;
   const unsigned *wimg = reinterpret_cast<const unsigned *>(g_smem + L.img + base);
   unsigned word = wimg[0];
-  float w0 =
-      s == 0 ? 0.0f : table_weight((int)(word & 0xffu), g_smem[L.img + base - L.mp + L.m - 1]);
+  double w0 =
+      s == 0 ? 0.0 : table_weight((int)(word & 0xffu), g_smem[L.img + base - L.mp + L.m - 1]);
   for (int k = s; k < e; k += 4)
   {
     const unsigned next = k + 4 < e     ? wimg[(k + 4 - s) >> 2]
                           : k + 4 < L.n ? *reinterpret_cast<const unsigned *>(
                                               g_smem + L.img + base + L.mp)
                                         : 0u;
-    float wl[4], wr[4];
+    double wl[4], wr[4];
     int I[5];
 #pragma unroll
     for (int t = 0; t < 4; ++t)
@@ -253,7 +263,7 @@ __device__ __forceinline__ void walk_chunks(const Line &L, int s, int e, int bas
 // Solves the line (rd, ri and img filled) and leaves the solution in rd
 // (depth) and ri (indicator).  Whole warp; every float element is rewritten
 // in place by the lane that owns it (the image bytes are read-only).
-__device__ __forceinline__ void solve_line(const Line &L, double lam)
+__device__ __forceinline__ void solve_line(const Line &L)
 {
   const int lane = threadIdx.x & 31;
   const int s = min(lane * L.m, L.n);
@@ -263,12 +273,12 @@ __device__ __forceinline__ void solve_line(const Line &L, double lam)
   // entries grow by at most 1 + 2*lambda per element, far inside the double
   // range for segments of <= 128 elements, so no per-step rescaling.
   Mat2 P{1.0, 0.0, 0.0, 1.0};
-  walk_chunks(L, s, e, base, [&](int, const float(&wl)[4], const float(&wr)[4]) {
+  walk_chunks(L, s, e, base, [&](int, const double(&wl)[4], const double(&wr)[4]) {
 #pragma unroll
     for (int t = 0; t < 4; ++t)
     {
-      const double a = -lam * (double)wl[t], c = -lam * (double)wr[t];
-      const double bb = 1.0 + lam * ((double)wl[t] + (double)wr[t]);
+      const double a = -wl[t], c = -wr[t];
+      const double bb = 1.0 + (wl[t] + wr[t]);
       P = Mat2{c * P.c, c * P.d, bb * P.c - a * P.a, bb * P.d - a * P.b};
     }
   });
@@ -294,21 +304,21 @@ __device__ __forceinline__ void solve_line(const Line &L, double lam)
   Mat2 Q{1.0, 0.0, 0.0, 1.0};
   double Dprev = 1.0;
   Aff F{1.0f, 0.0f, 0.0f};
-  walk_chunks(L, s, e, base, [&](int k, const float(&wl)[4], const float(&wr)[4]) {
+  walk_chunks(L, s, e, base, [&](int k, const double(&wl)[4], const double(&wr)[4]) {
     const int p = base + (k - s);
     const float4 rd = ld4(L.rd, p), ri = ld4(L.ri, p);
     float4 inv4;
 #pragma unroll
     for (int t = 0; t < 4; ++t)
     {
-      const double a = -lam * (double)wl[t], c = -lam * (double)wr[t];
-      const double bb = 1.0 + lam * ((double)wl[t] + (double)wr[t]);
+      const double a = -wl[t], c = -wr[t];
+      const double bb = 1.0 + (wl[t] + wr[t]);
       Q = Mat2{c * Q.c, c * Q.d, bb * Q.c - a * Q.a, bb * Q.d - a * Q.b};
       const double Dk = Q.c * z0 + Q.d;
       const float invf = (float)(Dprev * recip_pos(Dk));
       Dprev = Dk;
       set4(inv4, t, invf);
-      const float alpha = (float)(lam * (double)wl[t]) * invf;
+      const float alpha = (float)wl[t] * invf;
       F = Aff{alpha * F.g, alpha * F.hd + f4(rd, t) * invf, alpha * F.hi + f4(ri, t) * invf};
     }
     st4(L.cp, p, inv4);
@@ -329,7 +339,7 @@ __device__ __forceinline__ void solve_line(const Line &L, double lam)
   // -------- forward values of the segment, eliminated super-diagonal
   // c'_k = c_k / den_k, back-substitution composition
   Aff G{1.0f, 0.0f, 0.0f};
-  walk_chunks(L, s, e, base, [&](int k, const float(&wl)[4], const float(&wr)[4]) {
+  walk_chunks(L, s, e, base, [&](int k, const double(&wl)[4], const double(&wr)[4]) {
     const int p = base + (k - s);
     const float4 inv4 = ld4(L.cp, p);
     float4 rd = ld4(L.rd, p), ri = ld4(L.ri, p), cp4;
@@ -337,8 +347,8 @@ __device__ __forceinline__ void solve_line(const Line &L, double lam)
     for (int t = 0; t < 4; ++t)
     {
       const float invf = f4(inv4, t);
-      const float alpha = (float)(lam * (double)wl[t]) * invf;
-      const float cpk = (float)(-lam * (double)wr[t] * (double)invf);
+      const float alpha = (float)wl[t] * invf;
+      const float cpk = (float)(-wr[t] * (double)invf);
       dprev = alpha * dprev + f4(rd, t) * invf;
       iprev = alpha * iprev + f4(ri, t) * invf;
       set4(rd, t, dprev);
@@ -393,7 +403,7 @@ __global__ void __launch_bounds__(kMaxRowWarps * 32)
 {
   int lb;
   const JobDesc &J = job_of(B, lb);
-  build_weight_table<A>(kp.up_sigma);
+  build_weight_table<A>(kp.up_sigma, kp.up_lambda);
   __syncthreads();
   after_previous();
   const int W = J.W, H = J.H;
@@ -405,7 +415,8 @@ __global__ void __launch_bounds__(kMaxRowWarps * 32)
   const uint8_t *img = J.ref + (size_t)y * J.ref_pitch;
   const float w_close = (n < W) ? edge_weight<A>((float)img[n], (float)img[n - 1], kp.up_sigma)
                                 : (W % 16 != 0 ? 1.0f : 0.0f);
-  const Line L = line_at(kTableBytes + warp * line_bytes(max_n), n, w_close);
+  const Line L =
+      line_at(kTableBytes + warp * line_bytes(max_n), n, kp.up_lambda * (double)w_close);
   const float *sp = J.sparse + (size_t)y * W;
   // the row's fusion z-buffer keys start empty for this frame's fusion (the
   // previous frame's update left them set); coalesced stores in a
@@ -437,7 +448,7 @@ __global__ void __launch_bounds__(kMaxRowWarps * 32)
     }
   }
   __syncwarp();
-  solve_line(L, kp.up_lambda);
+  solve_line(L);
   float2 *out = J.rowres + (size_t)y * W;
   for (int k = lane; k < n; k += 32)
   {
@@ -452,20 +463,20 @@ __global__ void __launch_bounds__(kMaxColLines * 32)
 {
   int lb;
   const JobDesc &J = job_of(B, lb);
-  build_weight_table<A>(kp.up_sigma);
+  build_weight_table<A>(kp.up_sigma, kp.up_lambda);
   after_previous();
   const int W = J.W, H = J.H;
   const int warp = threadIdx.x >> 5;
   const int lines = blockDim.x >> 5;
   const int x0 = lb * lines;
   const int n = H / 8 * 8;
-  const int per_line = line_bytes(max_n);
+  const int per_line = stripe_pitch(max_n, lines);
   // cooperative stripe load: thread t owns column x0 + t % lines and rows
   // t / lines + 32 j (blockDim.x = 32 lines); a batch of loads per thread in
   // flight before their shared-memory stores
   const int kt = (int)threadIdx.x / lines, c = (int)threadIdx.x - kt * lines;
   const int xt = x0 + c;
-  const Line Lt = line_at(kTableBytes + c * per_line, n, 0.0f);
+  const Line Lt = line_at(kTableBytes + c * per_line, n, 0.0);
   if (xt < W)
   {
     const float2 *rsrc = J.rowres + (size_t)kt * W + xt;
@@ -505,7 +516,8 @@ __global__ void __launch_bounds__(kMaxColLines * 32)
         (n < H) ? edge_weight<A>((float)J.ref[(size_t)n * J.ref_pitch + x],
                                  (float)J.ref[(size_t)(n - 1) * J.ref_pitch + x], kp.up_sigma)
                 : (H % 16 != 0 ? 1.0f : 0.0f);
-    solve_line(line_at(kTableBytes + warp * per_line, n, w_close), kp.up_lambda);
+    solve_line(
+        line_at(kTableBytes + warp * per_line, n, kp.up_lambda * (double)w_close));
   }
   __syncthreads();
   if (xt < W)
@@ -527,7 +539,7 @@ size_t row_solve_smem(int max_w, int rows)
 }
 size_t col_solve_smem(int max_h, int lines)
 {
-  return (size_t)kTableBytes + (size_t)lines * line_bytes(max_h);
+  return (size_t)kTableBytes + (size_t)lines * stripe_pitch(max_h, lines);
 }
 
 void prepare_upsample_kernels()
