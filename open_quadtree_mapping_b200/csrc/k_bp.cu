@@ -9,9 +9,7 @@
 //
 // Lane groups: a cell is handled by a group of LPC lanes (32 for 96 and 128
 // hypotheses, 16 for 48 and 64, 8 for 32), so a warp updates 32/LPC cells at
-// once.  The half-sweeps hold four consecutive hypotheses per lane
-// (QuadLayout), the extraction the hypotheses g, g+LPC, g+2*LPC, ... in lane g
-// (HypLayout; every supported count is exactly LPC x 3 or 4).  The four
+// once; a lane holds four consecutive hypotheses (QuadLayout).  The four
 // directions are computed from one load of the data cost and the four incoming
 // messages.  The normalising sum uses the reference's stride-halving tree
 // (bpextract.cu:293-300) over the next power of two P >= D with zero padding.
@@ -41,59 +39,18 @@ constexpr __host__ __device__ int pow2_ceil(int n)
   return p;
 }
 
+// Lane g of a cell's group holds the four consecutive hypotheses 4 g .. 4 g + 3
+// (one 16-byte access per image; d +- 1 needs two shuffles per direction).  At
+// 48 and 96 hypotheses the last quarter of a group's lanes holds padding.
 template <int D>
-struct HypLayout
+struct QuadLayout
 {
-  static constexpr int P = pow2_ceil(D);              // tree width
-  static constexpr int LPC = P / 4 < 32 ? P / 4 : 32; // lanes per cell
-  static constexpr int NV = (D + LPC - 1) / LPC;      // register slots per lane
-  static constexpr int G = 32 / LPC;                  // cells per warp
-  static_assert(NV * LPC == D, "hypothesis count must fill the lane group");
+  static constexpr int P = pow2_ceil(D); // tree width
+  static constexpr int LPC = P / 4;      // lanes per cell
+  static constexpr int ACT = D / 4;      // lanes with hypotheses
+  static constexpr int G = 32 / LPC;     // cells per warp
+  static_assert(D % 4 == 0 && LPC <= 32, "a cell's hypotheses fill lanes of one warp");
 };
-
-template <int D>
-__device__ __forceinline__ void tree_argmin(const float (&v)[HypLayout<D>::NV], int gl,
-                                            float &best_v, int &best_i)
-{
-  constexpr int P = HypLayout<D>::P;
-  constexpr int NV = HypLayout<D>::NV;
-  constexpr int LPC = HypLayout<D>::LPC;
-  float a[NV];
-  int ai[NV];
-#pragma unroll
-  for (int k = 0; k < NV; ++k)
-  {
-    a[k] = v[k];
-    ai[k] = gl + LPC * k;
-  }
-#pragma unroll
-  for (int s = P / 2; s >= LPC; s /= 2)
-  {
-    const int t = s / LPC;
-#pragma unroll
-    for (int k = 0; k < t; ++k)
-      if (k + t < NV && a[k + t] < a[k])
-      {
-        a[k] = a[k + t];
-        ai[k] = ai[k + t];
-      }
-  }
-  float r = a[0];
-  int ri = ai[0];
-#pragma unroll
-  for (int o = LPC / 2; o > 0; o >>= 1)
-  {
-    const float ov = __shfl_down_sync(0xffffffffu, r, o, LPC);
-    const int oi = __shfl_down_sync(0xffffffffu, ri, o, LPC);
-    if (ov < r)
-    {
-      r = ov;
-      ri = oi;
-    }
-  }
-  best_v = r;
-  best_i = ri;
-}
 
 // sum / (float)DEPTH_NUM (bpextract.cu:302); D is a compile-time constant
 // here as DEPTH_NUM is in the reference.
@@ -211,18 +168,6 @@ __device__ __forceinline__ float4 msg_load(const float *p)
 {
   return *reinterpret_cast<const float4 *>(p);
 }
-
-// ---- layout of the half-sweeps: lane g of a cell's group holds the four
-// consecutive hypotheses 4 g .. 4 g + 3 (one 16-byte load per message image
-// instead of four 4-byte ones; d +- 1 needs two shuffles per direction instead
-// of eight).  Groups have P / 4 lanes, as above; at 48 and 96 hypotheses the
-// last quarter of a group's lanes holds padding.
-template <int D>
-struct QuadLayout
-{
-  static constexpr int P = HypLayout<D>::P, LPC = P / 4, ACT = D / 4;
-  static_assert(LPC == HypLayout<D>::LPC, "one group layout");
-};
 
 // One reduction step across lanes gl and gl ^ o that also halves the values a
 // lane holds: lanes with bit o clear go on with lo, the others with hi.
@@ -469,7 +414,7 @@ __global__ void __launch_bounds__(kMaxCellWarps * 32, 4)
                KParams kp)
 {
   after_previous();
-  constexpr int G = HypLayout<D>::G;
+  constexpr int G = QuadLayout<D>::G;
   int lb;
   const JobDesc &J = job_of(B, lb);
   if (J.D != D)
@@ -491,7 +436,7 @@ __global__ void __launch_bounds__(kMaxCellWarps * 32, 4)
                   const __grid_constant__ SweepIO io, KParams kp)
 {
   after_previous();
-  constexpr int G = HypLayout<D>::G;
+  constexpr int G = QuadLayout<D>::G;
   const LevelDesc &L = B.one.lv[level];
   const int item0 = ((int)blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5)) * G;
   if (item0 >= (L.w + 1) / 2 * L.h)
@@ -767,14 +712,70 @@ __global__ void __launch_bounds__(kCoarseMaxThreads, 1)
 }
 
 // ------------------------------------------------------------- extract
-// depth_extract (bpextract.cu:314-372), one lane group per level-0 cell.
+// The reference's stride-halving argmin (bpextract.cu:340-355) of
+// b[j] = value(4 g + j) over the group: a right element replaces the left one
+// only when strictly smaller.  Strides of four and more pair lanes; the first
+// two also share out the four j over the lanes, so strides 2 and 1 pair lanes
+// as well.  Padding must never be smaller than anything (infinity).  Every
+// lane ends with the result.
+template <int LPC>
+__device__ __forceinline__ void quad_argmin(const float (&b)[4], int gl, float &best_v, int &best_i)
+{
+  // lanes with bit o clear hold the left element
+  auto pick = [&](float own, int oi, float other, int ti, bool right, float &v, int &i) {
+    const float l = right ? other : own, r = right ? own : other;
+    const bool take = r < l;
+    v = take ? r : l;
+    i = take == right ? oi : ti;
+  };
+  const bool h1 = (gl & (LPC / 2)) != 0, h2 = (gl & (LPC / 4)) != 0;
+  const int mate = gl ^ (LPC / 2);
+  float v[2];
+  int i[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+  {
+    const float send = h1 ? b[j] : b[2 + j], keep = h1 ? b[2 + j] : b[j];
+    const float got = __shfl_xor_sync(0xffffffffu, send, LPC / 2);
+    const int jj = h1 ? 2 + j : j;
+    pick(keep, 4 * gl + jj, got, 4 * mate + jj, h1, v[j], i[j]);
+  }
+  float r;
+  int ri;
+  {
+    const float send = h2 ? v[0] : v[1], keep = h2 ? v[1] : v[0];
+    const int si = h2 ? i[0] : i[1], ki = h2 ? i[1] : i[0];
+    const float got = __shfl_xor_sync(0xffffffffu, send, LPC / 4);
+    const int gi = __shfl_xor_sync(0xffffffffu, si, LPC / 4);
+    pick(keep, ki, got, gi, h2, r, ri);
+  }
+  auto step = [&](int o) {
+    const float got = __shfl_xor_sync(0xffffffffu, r, o);
+    const int gi = __shfl_xor_sync(0xffffffffu, ri, o);
+    pick(r, ri, got, gi, (gl & o) != 0, r, ri);
+  };
+#pragma unroll
+  for (int o = LPC / 8; o > 0; o >>= 1)
+    step(o);
+  step(LPC / 2); // stride 2: j and j ^ 2
+  step(LPC / 4); // stride 1: j and j ^ 1
+  best_v = r;
+  best_i = ri;
+}
+
+// Extraction, one lane group per level-0 cell, 16 bytes per lane and image as
+// in the half-sweeps (five images read, 4 bytes per leaf written).
+// Measured, one hypothesis every 8 to 32 per lane -> four consecutive ones:
+// 32 x 752x480 x 64 180 -> 152 us, 8 x 1920x1080 x 128 457 -> 316 us, with the
+// half-sweeps' memory rate reached at 128 hypotheses (5.1 GB at most, less the
+// cells that are no leaf origin).
 template <int D, int ARITH>
 __global__ void __launch_bounds__(kMaxCellWarps * 32)
     k_extract(const __grid_constant__ Batch B)
 {
   after_previous();
-  using HL = HypLayout<D>;
-  constexpr int NV = HL::NV, LPC = HL::LPC, G = HL::G;
+  using QL = QuadLayout<D>;
+  constexpr int LPC = QL::LPC, G = 32 / LPC;
   int lb;
   const JobDesc &J = job_of(B, lb);
   if (J.D != D)
@@ -786,8 +787,8 @@ __global__ void __launch_bounds__(kMaxCellWarps * 32)
   if (cell0 >= w * h)
     return; // the whole warp
   const int cell = cell0 + lane / LPC;
-  bool act = cell < w * h;
   int x = 0, y = 0;
+  bool act = cell < w * h;
   if (act)
   {
     x = cell % w;
@@ -803,45 +804,29 @@ __global__ void __launch_bounds__(kMaxCellWarps * 32)
   }
   if (!__any_sync(0xffffffffu, act))
     return;
-  const size_t c = (size_t)cell;
-  float b[NV];
-#pragma unroll
-  for (int k = 0; k < NV; ++k)
-  {
-    const int d = gl + LPC * k;
-    float v = 0.0f;
-    if (act)
-    {
-      v = L.data[c * D + d];
-      if (x != 0)
-        v += L.msg[kRight][(c - 1) * D + d];
-      if (x != w - 1)
-        v += L.msg[kLeft][(c + 1) * D + d];
-      if (y != 0)
-        v += L.msg[kDown][(c - w) * D + d];
-      if (y != h - 1)
-        v += L.msg[kUp][(c + w) * D + d];
-    }
-    b[k] = v;
-  }
+  const bool on = act && (QL::ACT == LPC || gl < QL::ACT);
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const size_t c = (size_t)cell * D + 4 * gl;
+  auto msg = [&](int dir, bool has, long off) {
+    return on && has ? msg_load(L.msg[dir] + (c + off * D)) : zero;
+  };
+  const float4 dat = on ? *reinterpret_cast<const float4 *>(L.data + c) : zero;
+  const float4 fl = msg(kRight, x > 0, -1), fr = msg(kLeft, x < w - 1, 1);
+  const float4 fu = msg(kDown, y > 0, -w), fd = msg(kUp, y < h - 1, w);
+  // the reference's order: from the left, the right, above, below
+  float b[4] = {(((dat.x + fl.x) + fr.x) + fu.x) + fd.x, (((dat.y + fl.y) + fr.y) + fu.y) + fd.y,
+                (((dat.z + fl.z) + fr.z) + fu.z) + fd.z, (((dat.w + fl.w) + fr.w) + fu.w) + fd.w};
+  if (QL::ACT < LPC && gl >= QL::ACT)
+    b[0] = b[1] = b[2] = b[3] = __int_as_float(0x7f800000);
   float bmin;
   int best;
-  tree_argmin<D>(b, gl, bmin, best);
-  best = __shfl_sync(0xffffffffu, best, 0, LPC);
-  bmin = __shfl_sync(0xffffffffu, bmin, 0, LPC);
+  quad_argmin<LPC>(b, gl, bmin, best);
   // neighbours of the winner for the parabola
-  const int ip = best > 0 ? best - 1 : 0, in_ = best < D - 1 ? best + 1 : D - 1;
-  float pre = 0.0f, post = 0.0f;
-#pragma unroll
-  for (int k = 0; k < NV; ++k)
-  {
-    const float vp = __shfl_sync(0xffffffffu, b[k], ip % LPC, LPC);
-    const float vn = __shfl_sync(0xffffffffu, b[k], in_ % LPC, LPC);
-    if (ip / LPC == k)
-      pre = vp;
-    if (in_ / LPC == k)
-      post = vn;
-  }
+  auto at = [&](int d) {
+    const float lo = (d & 1) ? b[1] : b[0], hi = (d & 1) ? b[3] : b[2];
+    return __shfl_sync(0xffffffffu, (d & 2) ? hi : lo, d >> 2, LPC);
+  };
+  const float pre = at(best > 0 ? best - 1 : 0), post = at(best < D - 1 ? best + 1 : D - 1);
   if (gl != 0 || !act)
     return;
   float disparity = (float)best;
@@ -1021,11 +1006,11 @@ int bp_cells_per_warp(int d)
 {
   switch (d)
   {
-  case 32: return HypLayout<32>::G;
-  case 48: return HypLayout<48>::G;
-  case 64: return HypLayout<64>::G;
-  case 96: return HypLayout<96>::G;
-  case 128: return HypLayout<128>::G;
+  case 32: return QuadLayout<32>::G;
+  case 48: return QuadLayout<48>::G;
+  case 64: return QuadLayout<64>::G;
+  case 96: return QuadLayout<96>::G;
+  case 128: return QuadLayout<128>::G;
   default: return 1;
   }
 }
@@ -1116,15 +1101,7 @@ void launch_bp_coarse(const Batch &B, int j0, int jobs, int d, const CoarsePlan 
 
 void launch_extract(const Batch &B, int blocks, int d, int arith, cudaStream_t s, int warps)
 {
-  switch (d)
-  {
-  case 32: extract_d<32>(B, blocks, arith, warps, s); break;
-  case 48: extract_d<48>(B, blocks, arith, warps, s); break;
-  case 64: extract_d<64>(B, blocks, arith, warps, s); break;
-  case 96: extract_d<96>(B, blocks, arith, warps, s); break;
-  case 128: extract_d<128>(B, blocks, arith, warps, s); break;
-  default: break;
-  }
+  by_d(d, [&](auto dc) { extract_d<decltype(dc)::value>(B, blocks, arith, warps, s); });
 }
 
 } // namespace qm
