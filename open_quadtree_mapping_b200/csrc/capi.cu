@@ -274,8 +274,9 @@ struct SoftBp
     const int L = q.bp_levels, D = q.num_hyp;
     const qm::KParams kp = qm::kparams(q);
     const qm::Batch B = qm::stage::single(J);
-    for (int l = 1; l < L; ++l)
-      qm::launch_pyramid(B, cdiv_i((long)J.lv[l].w * J.lv[l].h * (D / 4), qm::kFlatThreads), l, s);
+    for (int l = 1; l < L; l += qm::kPyramidLevels)
+      qm::launch_pyramid(B, qm::pyramid_blocks(J.lv[l].w, J.lv[l].h), l,
+                         std::min(qm::kPyramidLevels, L - l), s);
     qm::CoarsePlan cp;
     std::memset(&cp, 0, sizeof(cp));
     cp.keep = 1;

@@ -71,9 +71,10 @@ std::vector<int> stage_blocks(const Shape &s, const JobLayout &lay, const qm_par
   const int D = s.D;
   b[st.qt()] = quadtree_blocks(s.W, s.H, p.qt_max_level);
   b[st.cost()] = cost_tiles(lay.lw[0], lay.lh[0]) * cuts.cost_split;
-  // pyramid and message kernels move float4 groups of hypotheses
-  for (int l = 1; l < L; ++l)
-    b[st.pyr(l)] = cdiv((long)lay.lw[l] * lay.lh[l] * (D / 4), kFlatThreads);
+  // one launch per kPyramidLevels levels, at the finest of them
+  for (int l = 1; l < L; l += kPyramidLevels)
+    b[st.pyr(l)] = pyramid_blocks(lay.lw[l], lay.lh[l]);
+  // the message kernel moves float4 groups of hypotheses
   for (int l = 0; l < L; ++l)
     b[st.inherit(l)] = cdiv((long)lay.lw[l] * lay.lh[l] * (D / 4), kFlatThreads);
   // BP cells per block of the half-sweeps and of the extraction
@@ -204,8 +205,10 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
   const int max_d = T.dvals.empty() ? 0 : T.dvals.back();
   all(kCost, st.cost(),
       [&](const Batch &b, int g) { launch_cost(b, g, ar, max_d, T.cuts.cost_split, s, T.tune.cost_blocks); });
-  for (int l = 1; l < L; ++l)
-    all(kPyramid, st.pyr(l), [&](const Batch &b, int g) { launch_pyramid(b, g, l, s); });
+  for (int l = 1; l < L; l += kPyramidLevels)
+    all(kPyramid, st.pyr(l), [&](const Batch &b, int g) {
+      launch_pyramid(b, g, l, std::min(kPyramidLevels, L - l), s);
+    });
   // BP, coarse to fine.  Per hypothesis count the top levels lc[..]..L-1 whose
   // cells are few (and which have two or more half-sweeps) run as one cluster
   // launch; below them each level runs job range by job range (message

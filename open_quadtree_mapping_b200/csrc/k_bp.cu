@@ -62,43 +62,76 @@ __device__ __forceinline__ float mean_of(float sum)
   return sum / (float)D;
 }
 
-// The three kernels below move whole float4 groups of hypotheses (D is a
+// The kernels below move whole float4 groups of hypotheses (D is a
 // multiple of 16 for every supported count, and every cell row starts on a
 // 16-byte boundary); each component keeps its own arithmetic.
 
 // ------------------------------------------------------------- pyramid
 // cost_distribute (bpextract.cu:169-198): L_l(x,y) = sum of the existing 2x2
-// children, x offset outer, y offset inner, starting from 0.
+// children, x offset outer, y offset inner, starting from 0; levels `level` ..
+// level + n - 1 from level - 1.  A block makes a tile of 4 x 4 cells of the
+// first, 2 x 2 of the second and one of the third from 8 x 8 finer cells; the
+// levels it has just made are read from shared memory.  A cell that a level
+// does not have adds 0 there, which changes no sum.
+// Bound: launches where few streams run (a launch per level took three where one
+// does: 640x480 x 48 BP alone 126 -> 122 us, one 160x128 keyframe 189 -> 184 us),
+// DRAM where many do (the finest data term is read once: 32 x 752x480 x 64 82 us
+// both ways, the finest level's 185 MB are most of it).
 __global__ void __launch_bounds__(kFlatThreads)
-    k_pyramid(const __grid_constant__ Batch B, int level)
+    k_pyramid(const __grid_constant__ Batch B, int level, int n)
 {
   after_previous();
   int lb;
   const JobDesc &J = job_of(B, lb);
-  const LevelDesc &Lf = J.lv[level - 1];
-  const LevelDesc &Lc = J.lv[level];
-  const int D4 = J.D / 4;
-  const long t = (long)lb * blockDim.x + threadIdx.x;
-  if (t >= (long)Lc.w * Lc.h * D4)
-    return;
-  const int cell = (int)(t / D4);
-  const int q = (int)(t - (long)cell * D4);
-  const int x = cell % Lc.w, y = cell / Lc.w;
-  const float4 *src = reinterpret_cast<const float4 *>(Lf.data);
-  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int jj = 0; jj < 2; ++jj)
-      if (2 * x + i < Lf.w && 2 * y + jj < Lf.h)
+  const int D4 = J.D / 4, tid = threadIdx.x;
+  __shared__ float4 s_a[16 * (kMaxHyp / 4)], s_b[4 * (kMaxHyp / 4)];
+  const int tiles = (J.lv[level].w + 3) / 4;
+  const int ty = lb / tiles, tx = lb - ty * tiles;
+  // cells [4 tx, 4 tx + side) x [4 ty, ..) of a level: v(x, y, q) sums the children
+  auto make = [&](const LevelDesc &L, int side, float4 *keep, auto &&child) {
+    for (int k = tid; k < side * side * D4; k += kFlatThreads)
+    {
+      const int c = k / D4, q = k - c * D4, lx = c % side, ly = c / side;
+      const int x = tx * side + lx, y = ty * side + ly;
+      float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (x < L.w && y < L.h)
       {
-        const float4 v = src[((size_t)(2 * y + jj) * Lf.w + (2 * x + i)) * D4 + q];
-        s.x += v.x;
-        s.y += v.y;
-        s.z += v.z;
-        s.w += v.w;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int jj = 0; jj < 2; ++jj)
+          {
+            const float4 v = child(x, y, lx, ly, i, jj, q);
+            s.x += v.x;
+            s.y += v.y;
+            s.z += v.z;
+            s.w += v.w;
+          }
+        reinterpret_cast<float4 *>(L.data)[((size_t)y * L.w + x) * D4 + q] = s;
       }
-  reinterpret_cast<float4 *>(Lc.data)[(size_t)cell * D4 + q] = s;
+      if (keep)
+        keep[k] = s;
+    }
+  };
+  const LevelDesc &F = J.lv[level - 1];
+  make(J.lv[level], 4, s_a, [&](int x, int y, int, int, int i, int jj, int q) {
+    const int fx = 2 * x + i, fy = 2 * y + jj;
+    return fx < F.w && fy < F.h
+               ? reinterpret_cast<const float4 *>(F.data)[((size_t)fy * F.w + fx) * D4 + q]
+               : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  });
+  if (n < 2)
+    return;
+  __syncthreads();
+  make(J.lv[level + 1], 2, s_b, [&](int, int, int lx, int ly, int i, int jj, int q) {
+    return s_a[((2 * ly + jj) * 4 + 2 * lx + i) * D4 + q];
+  });
+  if (n < 3)
+    return;
+  __syncthreads();
+  make(J.lv[level + 2], 1, nullptr, [&](int, int, int, int, int i, int jj, int q) {
+    return s_b[(jj * 2 + i) * D4 + q];
+  });
 }
 
 // The reference's quadtree test of the bp kernel (bpextract.cu:214-220): a
@@ -1015,10 +1048,11 @@ int bp_cells_per_warp(int d)
   }
 }
 
-void launch_pyramid(const Batch &B, int blocks, int level,
-                    cudaStream_t s)
+int pyramid_blocks(int w, int h) { return (w + 3) / 4 * ((h + 3) / 4); }
+
+void launch_pyramid(const Batch &B, int blocks, int level, int n, cudaStream_t s)
 {
-  launch_kernel(k_pyramid, blocks, kFlatThreads, 0, s, B.early, B, level);
+  launch_kernel(k_pyramid, blocks, kFlatThreads, 0, s, B.early, B, level, n);
 }
 
 void launch_msg_inherit(const Batch &B, int blocks, int level, int iters, int qt_max,

@@ -88,7 +88,11 @@ int cost_split(long tiles);
 // register budget
 void launch_cost(const Batch &B, int blocks, int arith, int max_d, int split, cudaStream_t s,
                  int blocks_per_sm = kCostBlocks);
-void launch_pyramid(const Batch &B, int blocks, int level, cudaStream_t s);
+// Data terms of the levels `level` .. level + n - 1 (n <= kPyramidLevels) from
+// level - 1; pyramid_blocks of level `level`'s size
+constexpr int kPyramidLevels = 3;
+int pyramid_blocks(int w, int h);
+void launch_pyramid(const Batch &B, int blocks, int level, int n, cudaStream_t s);
 // writes the inherited messages of level `level` that its sweeps will read
 // (cells the quadtree test skips; all unswept cells when iters < 2)
 void launch_msg_inherit(const Batch &B, int blocks, int level, int iters, int qt_max,
