@@ -100,6 +100,7 @@ struct StageTable
   std::vector<int> dvals;          // hypothesis counts present
   std::vector<size_t> level_bytes; // per job and BP level: data + messages
   std::vector<int> job_d;          // per job: hypothesis count
+  std::vector<int> job_slots;      // per job: measurement slots
   std::vector<long> level_cells;   // per job and BP level: cells
   int max_w = 0, max_h = 0;        // longest lines of the row / column solves
   Cuts cuts;                       // how the launch's work is cut
@@ -203,8 +204,18 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
   };
   all(kQuadtree, st.qt(), [&](const Batch &b, int g) { launch_quadtree(b, g, kp, s); });
   const int max_d = T.dvals.empty() ? 0 : T.dvals.back();
-  all(kCost, st.cost(),
-      [&](const Batch &b, int g) { launch_cost(b, g, ar, max_d, T.cuts.cost_split, s, T.tune.cost_blocks); });
+  // the cost blocks' work (hypotheses x slots) that is in jobs with much of it
+  long work = 0, much = 0;
+  for (int j = ja; j < jb; ++j)
+  {
+    const long each = (long)T.job_d[j] * T.job_slots[j] / T.cuts.cost_split;
+    const long all_blocks = each * (T.begin(st.cost(), j + 1) - T.begin(st.cost(), j));
+    work += all_blocks;
+    much += each >= kViewWork ? all_blocks : 0;
+  }
+  all(kCost, st.cost(), [&](const Batch &b, int g) {
+    launch_cost(b, g, ar, max_d, T.cuts.cost_split, 2 * much > work, s, T.tune.cost_blocks);
+  });
   for (int l = 1; l < L; l += kPyramidLevels)
     all(kPyramid, st.pyr(l), [&](const Batch &b, int g) {
       launch_pyramid(b, g, l, std::min(kPyramidLevels, L - l), s);
@@ -747,6 +758,7 @@ std::unique_ptr<TableBuf> Engine::build_table(const std::vector<int> &active, co
                               sizeof(float));
     for (int l = 0; l < L; ++l)
       T.level_cells.push_back((long)layouts_[j].lw[l] * layouts_[j].lh[l]);
+    T.job_slots.push_back(shapes_[j].F);
   }
   T.add_jobs(per_job, ds);
   const int ns = (int)T.uniform.size();
@@ -1179,6 +1191,7 @@ int run_range(const Batch &B, const Shape &s, const qm_params &p, int first, int
   StageTable T;
   T.cuts = Cuts::of(cost_tiles(lay.lw[0], lay.lh[0]), (long)s.W * s.H);
   T.add_jobs({stage_blocks(s, lay, p, T.tune, T.cuts)}, {s.D});
+  T.job_slots = {s.F};
   T.max_w = s.W;
   T.max_h = s.H;
   for (int l = 0; l < p.bp_levels; ++l)

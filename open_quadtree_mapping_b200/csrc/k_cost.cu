@@ -133,6 +133,66 @@ struct __align__(16) SlotParam
   unsigned weight;
 };
 
+// Hypotheses [lo, hi] (real numbers of the line 0 .. last, lo > hi: none) outside
+// of which a node's projection into a slot is certainly not in view.  With inverse
+// depth w the projected point is, up to scale, q(w) = R ray + t w, and in view
+// means (q_x / q_z, q_y / q_z) within four bounds: four linear forms in w that
+// are all >= 0 where q_z > 0, or all <= 0 where q_z < 0 (the projection does not
+// ask on which side of the camera the point lies).  Every form is widened by
+// kViewSlack of the sum of its terms' magnitudes (the rays are unit vectors), far
+// above what float rounding moves the compared coordinates by in either arithmetic
+// (a dozen roundings, 1e-6); a bound that comes out NaN does not narrow anything.
+constexpr float kViewSlack = 1e-5f;
+__device__ __forceinline__ void view_range(const float4 &t0, const float4 &t1, const float4 &t2,
+                                           const float3 &ray, const Cam &cam, float W, float H,
+                                           float w0, float dw, float last, int &first, int &end)
+{
+  const float ax = t0.x * ray.x + t0.y * ray.y + t0.z * ray.z;
+  const float ay = t1.x * ray.x + t1.y * ray.y + t1.z * ray.z;
+  const float az = t2.x * ray.x + t2.y * ray.y + t2.z * ray.z;
+  const float w_max = fmaxf(fabsf(w0), fabsf(w0 + dw * last));
+  const float slack = kViewSlack *
+                      (cam.fx + cam.fy + fabsf(cam.cx) + fabsf(cam.cy) + 2.0f * (W + H)) *
+                      (fabsf(t0.x) + fabsf(t0.y) + fabsf(t0.z) + fabsf(t1.x) + fabsf(t1.y) +
+                       fabsf(t1.z) + fabsf(t2.x) + fabsf(t2.y) + fabsf(t2.z) +
+                       (fabsf(t0.w) + fabsf(t1.w) + fabsf(t2.w)) * w_max);
+  float lo[2] = {0.0f, 0.0f}, hi[2] = {last, last};
+  // the form p + q w >= 0, and <= 0 for the points behind the camera
+  auto form = [&](float p, float q) {
+    const float a = p + q * w0, b = q * dw; // in the hypothesis index
+    const float inv = __fdividef(1.0f, b);
+#pragma unroll
+    for (int side = 0; side < 2; ++side)
+    {
+      const float c = (side ? -a : a) + slack, m = side ? -b : b;
+      const float at = (side ? c : -c) * inv;
+      if (m > 0.0f)
+        lo[side] = fmaxf(lo[side], at);
+      else if (m < 0.0f)
+        hi[side] = fminf(hi[side], at);
+      else if (c < 0.0f)
+        hi[side] = -1e9f;
+    }
+  };
+  auto axis = [&](float f, float c, float size, float p, float q) {
+    const float below = c - 1.25f, above = size - 2.25f - c; // a quarter pixel wide of the bounds
+    form(f * p + below * az, f * q + below * t2.w);
+    form(above * az - f * p, above * t2.w - f * q);
+  };
+  axis(cam.fx, cam.cx, W, ax, t0.w);
+  axis(cam.fy, cam.cy, H, ay, t1.w);
+  // a hypothesis to either side for the rounding of the bounds themselves
+  first = 1 << 20;
+  end = -1;
+#pragma unroll
+  for (int side = 0; side < 2; ++side)
+    if (!(lo[side] > hi[side] + 2.0f))
+    {
+      first = min(first, (int)floorf(fminf(lo[side], 1e6f)) - 1);
+      end = max(end, (int)ceilf(fminf(hi[side], 1e6f)) + 1);
+    }
+}
+
 // Share of the centres that must lie within the margin, else the slot's patches
 // are taken pixel by pixel at once: a deferred patch costs about 1.3 of those and
 // an aligned one 0.7, so the list pays up to about a quarter.  (Frames up to 18
@@ -158,8 +218,9 @@ constexpr int kCostWarps = kFlatThreads / 32;
 // 8 x 1920x1080 x 128, 20 slots 4.93 -> 4.36, one 1280x720, 10 slots 0.144 ->
 // 0.123, one 1920x1080 x 128, 18 slots 0.870 -> 0.689.
 // WORDS: the slot images' rows all start on a word, so that a patch's rows are
-// offset alike.
-template <class A, int MINB, bool WORDS>
+// offset alike.  VIEW: the hypotheses out of a slot's view are found first
+// (kViewWork).
+template <class A, int MINB, bool WORDS, bool VIEW>
 __global__ void __launch_bounds__(kFlatThreads, MINB)
     k_cost(const __grid_constant__ Batch B, int split)
 {
@@ -177,6 +238,10 @@ __global__ void __launch_bounds__(kFlatThreads, MINB)
   __shared__ unsigned s_row[3][kCostCells];
   __shared__ unsigned s_nodes;
   __shared__ int s_fast;
+  // hypotheses at which any node of the tile may be in view of a slot, and per
+  // hypothesis the slots
+  __shared__ int2 s_range[VIEW ? kMaxSlots : 1];
+  __shared__ unsigned s_view[VIEW ? kMaxHyp : 1];
   // per warp: patches to be taken pixel by pixel (position; node, hypothesis
   // and slot)
   __shared__ float4 s_late[kCostWarps][96];
@@ -259,6 +324,34 @@ __global__ void __launch_bounds__(kFlatThreads, MINB)
   // are floats, the comparisons exact; NaN fails)
   const float ulo = 1.5f, uhi = (float)W - 2.5f, vhi = (float)H - 2.5f;
   const unsigned bias = 0u - kBias * (pitch + 1u);
+  if constexpr (VIEW)
+  {
+    for (int f = warp; f < F; f += kCostWarps)
+    {
+      const int k = min(lane, n - 1);
+      int first = 1 << 20, end = -1;
+      if (n > 0)
+        view_range(s_pose[3 * f], s_pose[3 * f + 1], s_pose[3 * f + 2],
+                   make_float3(s_dir[0][k], s_dir[1][k], s_dir[2][k]), cam, (float)W, (float)H,
+                   (float)J.min_inv, (float)J.step, (float)(all_d - 1), first, end);
+      first = __reduce_min_sync(0xffffffffu, first);
+      end = __reduce_max_sync(0xffffffffu, end);
+      if (lane == 0)
+        s_range[f] = make_int2(first, end);
+    }
+    __syncthreads();
+    for (int d = tid; d < D; d += blockDim.x)
+    {
+      unsigned m = 0;
+      for (int f = 0; f < F; ++f)
+      {
+        const int2 r = s_range[f];
+        m |= (h0 + d >= r.x && h0 + d <= r.y ? 1u : 0u) << f;
+      }
+      s_view[d] = m;
+    }
+    __syncthreads();
+  }
   // Thread t evaluates node k = t % n at hypotheses g, g + per, g + 2 per,
   // ... (g = t / n, per = threads per node): consecutive lanes hold
   // neighbouring nodes at one depth, whose projections are neighbours in the
@@ -308,11 +401,23 @@ __global__ void __launch_bounds__(kFlatThreads, MINB)
       const bool on_a = mine && da < D, on_b = mine && db < D;
       const float3 pa = A::scale(dir, s_depth[min(da, D - 1)]);
       const float3 pb = A::scale(dir, s_depth[min(db, D - 1)]);
+      // the slots that any of the warp's pairs may be in view of
+      unsigned view = 0u;
+      if constexpr (VIEW)
+        view = __reduce_or_sync(0xffffffffu,
+                                (on_a ? s_view[da] : 0u) | (on_b ? s_view[db] : 0u));
       unsigned acc_a = 0, acc_b = 0;
       const unsigned id_a = ((unsigned)k << 8) | ((unsigned)da << 16);
       const unsigned id_b = ((unsigned)k << 8) | ((unsigned)db << 16);
       for (int f = 0; f < fast; ++f)
       {
+        if constexpr (VIEW)
+        {
+          const bool any = view & 1u;
+          view >>= 1;
+          if (!any)
+            continue;
+        }
         const float4 t0 = s_pose[3 * f], t1 = s_pose[3 * f + 1], t2 = s_pose[3 * f + 2];
         const SlotParam sp = s_slot[f];
         const float2 ua = project(t0, t1, t2, pa), ub = project(t0, t1, t2, pb);
@@ -375,6 +480,13 @@ __global__ void __launch_bounds__(kFlatThreads, MINB)
       }
       for (int f = fast; f < F; ++f)
       {
+        if constexpr (VIEW)
+        {
+          const bool any = view & 1u;
+          view >>= 1;
+          if (!any)
+            continue;
+        }
         const float4 t0 = s_pose[3 * f], t1 = s_pose[3 * f + 1], t2 = s_pose[3 * f + 2];
         const SlotParam sp = s_slot[f];
         const F2 a = pack2(t0.x, t1.x), b = pack2(t0.y, t1.y);
@@ -450,12 +562,14 @@ int cost_split(long tiles) { return tiles <= 148 ? 4 : tiles <= 444 ? 2 : 1; }
 namespace
 {
 template <int MINB, bool WORDS>
-void cost_minb(const Batch &B, int blocks, int arith, int split, size_t sm, cudaStream_t s)
+void cost_minb(const Batch &B, int blocks, int arith, int split, bool view, size_t sm,
+               cudaStream_t s)
 {
+  auto go = [&](auto k) { launch_kernel(k, blocks, kFlatThreads, sm, s, B.early, B, split); };
   if (arith == QM_ARITH_IEEE)
-    launch_kernel(k_cost<ArithIeee, MINB, WORDS>, blocks, kFlatThreads, sm, s, B.early, B, split);
+    view ? go(k_cost<ArithIeee, MINB, WORDS, true>) : go(k_cost<ArithIeee, MINB, WORDS, false>);
   else
-    launch_kernel(k_cost<ArithRef, MINB, WORDS>, blocks, kFlatThreads, sm, s, B.early, B, split);
+    view ? go(k_cost<ArithRef, MINB, WORDS, true>) : go(k_cost<ArithRef, MINB, WORDS, false>);
 }
 
 // Slot images whose rows all start on a word: always in the engine's frame
@@ -471,18 +585,18 @@ bool word_rows(const Batch &B)
 }
 } // namespace
 
-void launch_cost(const Batch &B, int blocks, int arith, int max_d, int split, cudaStream_t s,
-                 int blocks_per_sm)
+void launch_cost(const Batch &B, int blocks, int arith, int max_d, int split, bool view,
+                 cudaStream_t s, int blocks_per_sm)
 {
   const size_t sm = sizeof(unsigned) * kCostCells * (max_d / split + 1);
   if (!word_rows(B)) // single calls only: the default budget
-    cost_minb<kCostBlocks, false>(B, blocks, arith, split, sm, s);
+    cost_minb<kCostBlocks, false>(B, blocks, arith, split, view, sm, s);
   else if (blocks_per_sm == 3)
-    cost_minb<3, true>(B, blocks, arith, split, sm, s);
+    cost_minb<3, true>(B, blocks, arith, split, view, sm, s);
   else if (blocks_per_sm == 4)
-    cost_minb<4, true>(B, blocks, arith, split, sm, s);
+    cost_minb<4, true>(B, blocks, arith, split, view, sm, s);
   else
-    cost_minb<5, true>(B, blocks, arith, split, sm, s);
+    cost_minb<5, true>(B, blocks, arith, split, view, sm, s);
 }
 
 } // namespace qm
