@@ -406,14 +406,13 @@ __device__ __forceinline__ void bwd_cell(const DiffBpR<R> &a, int x, int y, int 
 // final messages; a cell that the quadtree test skips is never consumed
 // before the start of the level, its adjoint collects every reader's; and a
 // message to a skipped cell or out of the image has no reader at this level
-// (only the finer one's copy-down), so its cell clears it once consumed.  dL/dP1 and dL/dP2 leave a block as one atomic each.  Measured at
-// 752x480 with 64 hypotheses (34 half-sweeps): 0.395 -> 0.257 ms.
+// (only the finer one's copy-down), so its cell clears it once consumed.
+// dL/dP1 and dL/dP2 leave a block as one atomic each.  Measured at 752x480 with
+// 64 hypotheses (34 half-sweeps): 0.395 -> 0.257 ms.
 template <int D, class R>
 __global__ void __launch_bounds__(kDiffWarps * 32) k_bp_sweep_bwd(const DiffBpR<R> a)
 {
   after_previous();
-  using M = Real<R>;
-  constexpr int NV = (D + 31) / 32;
   __shared__ double s_gp[2][kDiffWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int w = a.w, h = a.h, hw = (w + 1) / 2;
