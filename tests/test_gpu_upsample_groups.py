@@ -9,7 +9,7 @@ from open_quadtree_mapping_b200.params import ARITH_IEEE, ARITH_REFERENCE, Param
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [(16, 8), (48, 24), (144, 136), (752, 480), (1000, 520), (1040, 1032), (1920, 1080)]
+SIZES = [(16, 8), (48, 24), (144, 136), (752, 480), (1008, 520), (1040, 1032), (1920, 1080)]
 
 
 @pytest.mark.parametrize("arith", [ARITH_IEEE, ARITH_REFERENCE])
@@ -26,5 +26,4 @@ def test_groups_equal_single_samples(W, H, arith, gpu):
     off.copy_(img)
     p = Params.for_range(64, 0.5, 50.0, arith=arith)
     a, b = stages.upsample(sparse, img, p), stages.upsample(sparse, off, p)
-    n = W // 16 * 16  # the row pass solves whole sixteens
-    assert torch.equal(a[:, :n].view(torch.int32), b[:, :n].view(torch.int32))
+    assert torch.equal(a.view(torch.int32), b.view(torch.int32))
