@@ -26,9 +26,6 @@ struct CudaError
   std::string msg;
 };
 
-// throws CudaError on failure
-void check(cudaError_t e, const char *what);
-
 // Kernel kinds, for per-kind timing (qm_batch_profile).
 enum KernelKind
 {

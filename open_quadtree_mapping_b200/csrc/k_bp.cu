@@ -915,7 +915,9 @@ bool coarse_prepare(int ctas)
   if (!(done.load(std::memory_order_acquire) & bit))
   {
     const auto k = k_bp_coarse<D, ARITH, HIST>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem - 64);
+    check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               kMaxBlockSmem - 64),
+          "BP cluster kernel");
     cudaLaunchConfig_t c = {};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -927,11 +929,13 @@ bool coarse_prepare(int ctas)
     c.attrs = at;
     c.numAttrs = 1;
     int clusters = 0;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-            cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&clusters, k, &c) == cudaSuccess && clusters > 0)
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveClusters(&clusters, k, &c);
+    if (e == cudaSuccess && clusters > 0)
       wide.fetch_or(bit, std::memory_order_acq_rel);
-    cudaGetLastError(); // a device without such clusters is no error
+    else if (e != cudaSuccess)
+      cudaGetLastError(); // a device without such clusters is no error
     done.fetch_or(bit, std::memory_order_acq_rel);
   }
   return ctas <= 8 || (wide.load(std::memory_order_acquire) & bit);
@@ -954,7 +958,7 @@ void coarse_k(const Batch &B, int j0, int jobs, const CoarsePlan &plan, KParams 
   c.stream = s;
   c.attrs = at;
   c.numAttrs = B.early ? 2 : 1;
-  cudaLaunchKernelEx(&c, k_bp_coarse<D, ARITH, HIST>, B, j0, plan, kp);
+  check(cudaLaunchKernelEx(&c, k_bp_coarse<D, ARITH, HIST>, B, j0, plan, kp), "kernel launch");
 }
 
 template <int D>

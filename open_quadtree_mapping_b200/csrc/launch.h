@@ -12,6 +12,9 @@
 namespace qm
 {
 
+// throws CudaError (engine.h) on failure
+void check(cudaError_t e, const char *what);
+
 // Launches a kernel that starts with after_previous().  early: its blocks may be
 // set up while the kernel before it in the stream still runs, which hides the
 // launch's own latency.  For one stream's work or one keyframe's: with several
@@ -33,7 +36,7 @@ void launch_kernel(void (*k)(P...), int blocks, int threads, size_t smem, cudaSt
   c.stream = s;
   c.attrs = at;
   c.numAttrs = early ? 1 : 0;
-  cudaLaunchKernelEx(&c, k, std::forward<A>(args)...);
+  check(cudaLaunchKernelEx(&c, k, std::forward<A>(args)...), "kernel launch");
 }
 
 // threads per block of the flat per-element kernels
