@@ -514,6 +514,7 @@ void StreamSet::step(const std::vector<int> &which, const uint8_t *const *imgs,
   {
     eng_->launch(active, ev_in_);
     last_active_ = active;
+    last_dense_parity_ = p;
   }
   check(cudaStreamWaitEvent(eng_->stream(), ev_up_[p], 0), "event wait");
   for (size_t k = 0; k < which.size(); ++k)
@@ -595,6 +596,9 @@ void StreamSet::run_resident()
   if (last_active_ != all)
     throw CudaError{QM_ERR_STATE, "every stream must have produced a depth map once"};
   wait();
+  // steps without a dense pass (semi2dense_ratio) flip the parity, but leave
+  // the last pass's slot tables in the block of its own
+  eng_->set_parity(last_dense_parity_);
   eng_->run(all);
   for (auto &s : st_)
     s.out_parity = eng_->parity();

@@ -149,7 +149,8 @@ private:
   int device_;
   std::vector<State> st_;
   std::unique_ptr<Engine> eng_;
-  std::vector<int> last_active_;
+  std::vector<int> last_active_; // streams of the last dense pass, and its parity
+  int last_dense_parity_ = 0;
   std::mutex mu_;
   // pipelining: uploads and downloads run on their own streams, branch by
   // branch (ev_in_: a branch's frames are up); per step
