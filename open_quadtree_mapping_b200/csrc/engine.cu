@@ -234,18 +234,17 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
   {
     const int d = T.dvals[di];
     long cells[kMaxLevels] = {};
-    int jobs = 0;
+    bool any = false;
     for (int j = ja; j < jb; ++j)
       if (T.job_d[j] == d)
       {
-        ++jobs;
+        any = true;
         for (int l = 0; l < L; ++l)
           cells[l] = std::max(cells[l], T.level_cells[(size_t)j * L + l]);
       }
     CoarsePlan cp;
     std::memset(&cp, 0, sizeof(cp));
-    if (jobs == 0 ||
-        !coarse_plan(cp, d, cells, L, p.bp_iters, coarse_cells, jobs, ar))
+    if (!any || !coarse_plan(cp, d, cells, L, p.bp_iters, coarse_cells, B.njobs, ar))
       continue;
     lc[di] = cp.lo;
     launch(kSweep, [&] { launch_bp_coarse(B, ja, jb - ja, d, cp, kp, ar, s); });

@@ -903,14 +903,16 @@ void sweep_d(const Batch &B, int blocks, int level, int parity, int first, int i
 }
 
 // Opt-ins of one k_bp_coarse instance on the current device (large shared
-// memory, clusters of 16); true when the device can hold such a cluster.
+// memory, clusters of 16); returns how many clusters of 16 full blocks the
+// device runs at once (0: it has none; a B200 runs 7).
 template <int D, int ARITH, bool HIST>
-bool coarse_prepare(int ctas)
+int coarse_prepare()
 {
-  static std::atomic<unsigned long long> done{0}, wide{0};
+  static std::atomic<unsigned long long> done{0};
+  static std::atomic<int> wide[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess)
-    return false;
+    return 0;
   const unsigned long long bit = 1ull << (dev & 63);
   if (!(done.load(std::memory_order_acquire) & bit))
   {
@@ -932,19 +934,21 @@ bool coarse_prepare(int ctas)
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveClusters(&clusters, k, &c);
-    if (e == cudaSuccess && clusters > 0)
-      wide.fetch_or(bit, std::memory_order_acq_rel);
-    else if (e != cudaSuccess)
+    if (e != cudaSuccess)
+    {
       cudaGetLastError(); // a device without such clusters is no error
+      clusters = 0;
+    }
+    wide[dev & 63].store(clusters, std::memory_order_relaxed);
     done.fetch_or(bit, std::memory_order_acq_rel);
   }
-  return ctas <= 8 || (wide.load(std::memory_order_acquire) & bit);
+  return wide[dev & 63].load(std::memory_order_relaxed);
 }
 
 template <int D, int ARITH, bool HIST>
 void coarse_k(const Batch &B, int j0, int jobs, const CoarsePlan &plan, KParams kp, cudaStream_t s)
 {
-  coarse_prepare<D, ARITH, HIST>(plan.ctas);
+  coarse_prepare<D, ARITH, HIST>();
   cudaLaunchConfig_t c = {};
   cudaLaunchAttribute at[2];
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -974,18 +978,22 @@ void coarse_d(const Batch &B, int j0, int jobs, const CoarsePlan &plan, KParams 
               : coarse_k<D, R, false>(B, j0, jobs, plan, kp, s);
 }
 
+// clusters of 16 blocks that run at once, as coarse_prepare
 template <int D>
-bool coarse_fit_d(CoarsePlan &plan, long cells, int ctas, bool shared_sm, int arith)
+int coarse_wide_d(bool keep, int arith)
 {
   constexpr int R = QM_ARITH_REFERENCE, I = QM_ARITH_IEEE;
+  if (arith == QM_ARITH_IEEE)
+    return keep ? coarse_prepare<D, I, true>() : coarse_prepare<D, I, false>();
+  return keep ? coarse_prepare<D, R, true>() : coarse_prepare<D, R, false>();
+}
+
+template <int D>
+bool coarse_fit_d(CoarsePlan &plan, long cells, int ctas, bool shared_sm)
+{
   const long per = (cells + ctas - 1) / ctas;
   constexpr size_t room = kMaxBlockSmem - 64; // 64: s_len
   if (per > 4096 || coarse_smem<D>((int)per, false) > room)
-    return false;
-  const bool can = arith == QM_ARITH_IEEE
-                       ? (plan.keep ? coarse_prepare<D, I, true>(ctas) : coarse_prepare<D, I, false>(ctas))
-                       : (plan.keep ? coarse_prepare<D, R, true>(ctas) : coarse_prepare<D, R, false>(ctas));
-  if (!can)
     return false;
   plan.ctas = ctas;
   plan.per = (int)per;
@@ -1110,19 +1118,22 @@ bool coarse_plan(CoarsePlan &plan, int d, const long *cells, int levels, const i
   plan.hi = levels - 1;
   for (int l = 0; l < levels; ++l)
     plan.iters[l] = iters[l];
-  // Few jobs: the widest cluster for each (a half-sweep's latency counts).
-  // Above kCoarseWideJobs clusters of 16 no longer run all at once (148 SMs);
-  // then 8 blocks of 512 threads per job, two on an SM, if the level fits them
-  // (32 x 752x480, all half-sweeps: 0.965 ms; one 1024-thread block per SM
-  // 1.055, the former launch 0.985).
-  const int first = jobs <= kCoarseWideJobs ? kCoarseMaxCtas : 8;
+  // As wide a cluster for each job as lets those of all jobs run at once: 16
+  // blocks of 1024 threads (a half-sweep's latency counts), above what the
+  // device holds of these 16 of 512, two on an SM, if the level fits them so,
+  // and above twice as many 8 of 512.  Measured (resident pass, 16 of 1024 / 16
+  // of 512 / 8 of 512): 160x128 x 64, 8 streams 215 / 161 / 171 us, 12 225 / 172
+  // / 181, 16 294 / 236 / 198; 320x240 8 267 / 255 / 272, 12 331 / 306 / 316;
+  // 752x480 12 951 / 943 / 937, 24 1858 / 1809 / 1783.
   for (int l = levels - 1; l >= 0 && iters[l] >= 2 && cells[l] <= max_cells; --l)
   {
     bool ok = false;
     by_d(d, [&](auto dc) {
       constexpr int D = decltype(dc)::value;
-      ok = coarse_fit_d<D>(plan, cells[l], first, first == 8, arith) ||
-           coarse_fit_d<D>(plan, cells[l], first == 8 ? kCoarseMaxCtas : 8, first == 8, arith);
+      const int wide = coarse_wide_d<D>(plan.keep != 0, arith);
+      const int first = jobs <= 2 * wide ? kCoarseMaxCtas : 8;
+      for (int ctas : {first, kCoarseMaxCtas + 8 - first})
+        ok = ok || ((ctas <= 8 || wide > 0) && coarse_fit_d<D>(plan, cells[l], ctas, jobs > wide));
     });
     if (!ok)
       break;

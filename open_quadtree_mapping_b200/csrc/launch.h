@@ -145,7 +145,6 @@ void launch_bp_sweep_io(const Batch &B, int d, int level, int it, const SweepIO 
 // level in shared memory, `per` cells per block.
 constexpr int kCoarseMaxThreads = 1024;
 constexpr int kCoarseMaxCtas = 16; // above the portable 8: asked of the device
-constexpr int kCoarseWideJobs = 8; // jobs that get clusters of 16 blocks
 struct CoarsePlan
 {
   int lo, hi;
@@ -155,10 +154,10 @@ struct CoarsePlan
   int keep;      // 1: the half-sweeps keep their states in hist
   HistLevel hist[kMaxLevels];
 };
-// Sizes the plan for `jobs` jobs of d hypotheses: the top levels with at most
-// max_cells cells in every job (cells[l]: the most), two half-sweeps or more,
-// and room in a cluster's shared memory.  False: no such level.  plan.keep is
-// read, the rest (but hist) written.
+// Sizes the plan for jobs of d hypotheses, `jobs` jobs of any count and of all
+// branches running at once: the top levels with at most max_cells cells in every
+// job (cells[l]: the most), two half-sweeps or more, and room in a cluster's shared
+// memory.  False: no such level.  plan.keep is read, the rest (but hist) written.
 bool coarse_plan(CoarsePlan &plan, int d, const long *cells, int levels, const int *iters,
                  long max_cells, int jobs, int arith);
 // jobs j0 .. j0 + jobs - 1 of the batch (B.jobs null: the inline job)
