@@ -319,7 +319,9 @@ __device__ __forceinline__ void cell_update(const float4 &dat, const float4 &fu,
     if (pad)
       low[dir] = FLT_MAX;
   }
-  const float cap = dir_min<LPC>(low, gl) + kp.P2;
+  // a cell without a finite value counts as FLT_MAX (infinite costs then give
+  // the same messages at every count, with padding lanes or without)
+  const float cap = fminf(dir_min<LPC>(low, gl), FLT_MAX) + kp.P2;
 #pragma unroll
   for (int dir = 0; dir < 4; ++dir)
   {
