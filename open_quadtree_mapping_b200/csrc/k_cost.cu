@@ -152,7 +152,8 @@ __device__ __forceinline__ void view_range(const float4 &t0, const float4 &t1, c
   const float az = t2.x * ray.x + t2.y * ray.y + t2.z * ray.z;
   const float w_max = fmaxf(fabsf(w0), fabsf(w0 + dw * last));
   const float slack = kViewSlack *
-                      (cam.fx + cam.fy + fabsf(cam.cx) + fabsf(cam.cy) + 2.0f * (W + H)) *
+                      (fabsf(cam.fx) + fabsf(cam.fy) + fabsf(cam.cx) + fabsf(cam.cy) +
+                       2.0f * (W + H)) *
                       (fabsf(t0.x) + fabsf(t0.y) + fabsf(t0.z) + fabsf(t1.x) + fabsf(t1.y) +
                        fabsf(t1.z) + fabsf(t2.x) + fabsf(t2.y) + fabsf(t2.z) +
                        (fabsf(t0.w) + fabsf(t1.w) + fabsf(t2.w)) * w_max);
