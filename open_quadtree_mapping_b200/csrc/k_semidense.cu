@@ -46,7 +46,7 @@ namespace
 {
 
 constexpr int kSdThreads = 256;
-constexpr int kSdTile = 1024; // most pixels of one block of the stereo update
+constexpr int kSdSmallTile = 256, kSdTile = 1024; // pixels of one block of the stereo update
 constexpr unsigned long long kSdEmpty = ~0ull;
 
 // reference constants (stereo_parameter.cuh:1-41)
@@ -570,33 +570,36 @@ __device__ __forceinline__ void update_seed(const SdJob &J, int x, int y, Fl<I> 
 // per seed; reads and writes only its own seed.
 // Bound: the search loop (up to 101 samples per observed seed, each a texture
 // fetch and about 60 instructions).  A block first collects the pixels of its
-// tile that will be searched, so that the warps of the loop are full (on
-// textured frames about half of the pixels pass the gates, scattered, and
-// almost every warp of consecutive pixels had some).  Nine streams of 624x408
-// to 1264x816: the step 1.37 -> 0.84 ms without the neighbourhood passes.
+// tile that will be searched, with what their gates computed, so that the warps
+// of the loop are full (on textured frames about half of the pixels pass the
+// gates, scattered, and almost every warp of consecutive pixels had some).
+// TILE: see sd_tile.  The step of one frame, a thread per pixel -> this, textured
+// views: 752x480 225 -> 209 us, 1280x720 374 -> 312, 1920x1080 677 -> 515; noise,
+// where every pixel is searched: 242 -> 242, 443 -> 441, 920 -> 929.
 // 4 blocks per SM (at most 64 registers instead of 86 / 102, i.e. 2 blocks):
 // the search loop is latency-bound, and the extra resident warps outweigh
 // the spilled values (tracker per stream and frame at 752x480: 0.171 ms at
 // 2 blocks, 0.144 at 3, 0.127 at 4, 0.125 at 5).
-template <bool I>
+template <bool I, int TILE>
 __global__ void __launch_bounds__(kSdThreads, 4) k_sd_update(const __grid_constant__ SdBatch B)
 {
   using F = Fl<I>;
-  __shared__ unsigned short s_list[kSdTile];
+  __shared__ float4 s_gates[TILE]; // gradient_max, gae, epi of a collected pixel
+  __shared__ unsigned short s_list[TILE];
   __shared__ int s_count;
   int lb;
   const SdJob &J = sd_job(B, B.tile_prefix, lb);
   if (J.mode < kSdUpdate)
     return; // the whole block
-  const int W = J.W, n = W * J.H, tile = B.tile, base = lb * tile;
+  const int W = J.W, n = W * J.H, base = lb * TILE;
   if (threadIdx.x == 0)
     s_count = 0;
   __syncthreads();
-  F gradient_max, gae;
-  float2 epi;
   const int lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < tile; i += kSdThreads)
+  for (int i = threadIdx.x; i < TILE; i += kSdThreads)
   {
+    F gradient_max, gae;
+    float2 epi;
     const int p = base + i, y = p / W, x = p - y * W;
     const bool on = p < n && observable<I>(J, x, y, gradient_max, gae, epi);
     const unsigned m = __ballot_sync(0xffffffffu, on);
@@ -605,15 +608,19 @@ __global__ void __launch_bounds__(kSdThreads, 4) k_sd_update(const __grid_consta
       at = atomicAdd(&s_count, __popc(m));
     at = __shfl_sync(0xffffffffu, at, 0);
     if (on)
-      s_list[at + __popc(m & ((1u << lane) - 1u))] = (unsigned short)i;
+    {
+      at += __popc(m & ((1u << lane) - 1u));
+      s_list[at] = (unsigned short)i;
+      s_gates[at] = make_float4(gradient_max.v, gae.v, epi.x, epi.y);
+    }
   }
   __syncthreads();
   const int count = s_count;
   for (int i = threadIdx.x; i < count; i += kSdThreads)
   {
     const int p = base + s_list[i], y = p / W, x = p - y * W;
-    observable<I>(J, x, y, gradient_max, gae, epi);
-    update_seed<I>(J, x, y, gradient_max, gae, epi);
+    const float4 g = s_gates[i];
+    update_seed<I>(J, x, y, F(g.x), F(g.y), make_float2(g.z, g.w));
   }
 }
 
@@ -919,7 +926,10 @@ void sd_sequence(const SdBatch &B, int blocks, int tiles, cudaStream_t s)
   k_sd_init<<<blocks, kSdThreads, 0, s>>>(B);
   // update_keyframe (seed_matrix.cu:401-446): stereo update, hole filling,
   // regularisation, projection into the incoming frame
-  k_sd_update<I><<<tiles, kSdThreads, 0, s>>>(B);
+  if (B.tile == kSdTile)
+    k_sd_update<I, kSdTile><<<tiles, kSdThreads, 0, s>>>(B);
+  else
+    k_sd_update<I, kSdSmallTile><<<tiles, kSdThreads, 0, s>>>(B);
   k_sd_fill<I><<<blocks, kSdThreads, 0, s>>>(B, 0, kSdUpdate);
   k_sd_regularize<I><<<blocks, kSdThreads, 0, s>>>(B, 1, 0, kSdUpdate);
   k_sd_project<I><<<blocks, kSdThreads, 0, s>>>(B);
@@ -939,10 +949,12 @@ void sd_sequence(const SdBatch &B, int blocks, int tiles, cudaStream_t s)
 int sd_blocks(int W, int H) { return (W * H + kSdThreads - 1) / kSdThreads; }
 
 // Larger tiles fill the warps of the search better; a step of few pixels needs
-// the blocks more: below two waves of blocks (148 SMs x 4) the tiles are
-// halved (one 752x480 stream 122 us per step against 132 at 1024 pixels; nine
-// streams with 4.9 M pixels 836 us at 1024 against 874 at 512, 849 at 2048).
-int sd_tile(long pixels) { return pixels < 2L * 592 * kSdTile ? kSdTile / 2 : kSdTile; }
+// the blocks more.  One frame, 256 / 512 / 1024 pixels a block: textured 320x240
+// 124 / 136 / 150 us, 752x480 208 / 212 / 230, 1280x720 312 / 315 / 318, 1920x1080
+// 549 / 535 / 515; noise 752x480 241 / 264 / 286, 1280x720 441 / 451 / 476,
+// 1920x1080 912 / 910 / 929.  The line lies at two waves of blocks of the large
+// tile (148 SMs x 4).
+int sd_tile(long pixels) { return pixels < 2L * 592 * kSdTile ? kSdSmallTile : kSdTile; }
 
 int sd_tiles(int W, int H, int tile) { return (W * H + tile - 1) / tile; }
 
