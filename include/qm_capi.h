@@ -201,7 +201,10 @@ int qm_batch_set_semidense(qm_batch *b, int enable);
  * latency-bound stages -- coarse BP levels, line solves -- with the others'
  * work); 1 = one sequence over all of them; default 3.  With k >= 2 streams
  * of different hypothesis counts get branches of their own, up to 4 in all.
- * Results do not depend on it. */
+ * Results do not depend on it.  A batch of several streams runs its branches at
+ * falling stream priorities above the default one, so its kernels are scheduled
+ * before the caller's own work on streams of default priority; a batch of one
+ * stream and a qm_depthmap run at the default. */
 int qm_batch_set_branches(qm_batch *b, int branches);
 /* L2 budget, in bytes, of a job range of the belief propagation: each BP
  * level runs over consecutive streams whose level costs and messages fit in

@@ -569,11 +569,13 @@ Engine::Engine(int device, const qm_params &p, const std::vector<Shape> &shapes)
   // results leave while the others still compute.  Measured with three
   // branches, equal priorities -> these: 32 x 752x480 submit + wait 3.98 ->
   // 3.32 ms, resident 2.53 -> 2.50; 8 x 1920x1080 10.3 -> 9.5, 8.98 -> 8.88.
+  // One stream has one branch: it stays at the default, beside the caller's own
+  // work.
   int low = 0, high = 0;
   check(cudaDeviceGetStreamPriorityRange(&low, &high), "stream priorities");
   auto make = [&](cudaStream_t *s, int i) {
-    check(cudaStreamCreateWithPriority(s, cudaStreamNonBlocking,
-                                       std::max(high, low - (kMaxBranches - 1 - i))),
+    const int raised = shapes.size() > 1 ? kMaxBranches - 1 - i : 0;
+    check(cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, std::max(high, low - raised)),
           "cudaStreamCreate");
   };
   make(&stream_, 0);
