@@ -216,8 +216,9 @@ int qm_batch_set_group_bytes(qm_batch *b, size_t bytes);
  * their half-sweeps in one launch, a cluster of blocks per stream with a
  * hardware cluster barrier between half-sweeps, instead of one launch per
  * half-sweep as the reference's bp_extract (bpextract.cu:122-143).  0 = one
- * launch per half-sweep everywhere; default 4096.  Results do not depend on
- * it. */
+ * launch per half-sweep everywhere.  Until it is called the library chooses:
+ * up to 1024 cells at 96 and 128 hypotheses, 2048 at 48 and 64, 4096 at 32, and
+ * twice as many where 2 to 7 streams run.  Results do not depend on it. */
 int qm_batch_set_coarse_bp(qm_batch *b, int max_cells);
 /* 1 = with two or more branches, branch i + 1 starts once branch i's cost
  * volume is done, so the issue-bound cost kernel of one branch overlaps the

@@ -287,7 +287,7 @@ struct SoftBp
       cp.hist[l] = hist_level(l);
     }
     int lc = L;
-    if (qm::coarse_plan(cp, D, cells, L, q.bp_iters, QM_DEFAULT_COARSE_CELLS, 1, q.arith))
+    if (qm::coarse_plan(cp, D, cells, L, q.bp_iters, qm::kCoarseAuto, 1, q.arith))
     {
       lc = cp.lo;
       qm::launch_bp_coarse(B, 0, 1, D, cp, kp, q.arith, s);

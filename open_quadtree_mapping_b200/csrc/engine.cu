@@ -229,7 +229,7 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
   auto any_of = [&](int d, int j0, int j1) {
     return std::find(T.job_d.begin() + j0, T.job_d.begin() + j1, d) != T.job_d.begin() + j1;
   };
-  const bool coarse = coarse_cells > 0 && in(st.sweep(L - 1));
+  const bool coarse = coarse_cells != 0 && in(st.sweep(L - 1));
   for (size_t di = 0; coarse && di < T.dvals.size(); ++di)
   {
     const int d = T.dvals[di];
@@ -1197,7 +1197,7 @@ int run_range(const Batch &B, const Shape &s, const qm_params &p, int first, int
   T.max_h = s.H;
   for (int l = 0; l < p.bp_levels; ++l)
     T.level_cells.push_back((long)lay.lw[l] * lay.lh[l]);
-  return enqueue_range(B, T, p, 0, QM_DEFAULT_COARSE_CELLS, first, last, stream);
+  return enqueue_range(B, T, p, 0, kCoarseAuto, first, last, stream);
 }
 
 int first_of(const char *name, int L)

@@ -52,16 +52,6 @@ enum KernelKind
 // 5.23 ms at 24 MiB).
 constexpr size_t kDefaultGroupBytes = 0;
 
-// Default coarse-level threshold of the BP: the top pyramid levels whose
-// largest cell count over the active jobs is at most this run all their
-// half-sweeps in one cluster launch (k_bp_coarse) instead of one launch per
-// half-sweep; 0 disables it.  4096 takes levels 2 and 3 of a 752x480 or
-// 1280x720 keyframe (1410 / 360 and 3600 / 920 cells) and level 3 of a
-// 1920x1080 one.
-#ifndef QM_DEFAULT_COARSE_CELLS
-#define QM_DEFAULT_COARSE_CELLS 4096
-#endif
-
 // Default number of concurrent pipeline branches per batch (consecutive ranges
 // of the active jobs, bit-identical results).  submit + wait / resident, two
 // and three branches: 32 x 752x480 3.45 / 2.48 and 3.32 / 2.50 ms, 8 x 752x480
@@ -195,14 +185,15 @@ public:
   int branches() const { return branches_; }
   size_t group_bytes() const { return group_bytes_; }
   // coarse BP levels (at most `cells` cells in every active job) in one
-  // cluster launch; 0: one launch per half-sweep at every level.  Results
-  // do not depend on it.
+  // cluster launch; 0: one launch per half-sweep at every level; kCoarseAuto
+  // until it is called.  Results do not depend on it.
   void set_coarse_cells(int cells) { coarse_cells_ = cells < 0 ? 0 : cells; }
   // true: branch i + 1 starts once branch i's cost volume is done, so the
   // issue-bound cost kernel of one branch runs beside the bandwidth-bound
-  // BP of the previous one; false (the default; measured faster on a B200:
-  // 2.91 vs 2.97 ms per 32 x 752x480 batch with two branches): all
-  // branches start together.  Results do not depend on it.
+  // BP of the previous one; false (the default; resident pass with three
+  // branches, off / on: 4 x 752x480 401 / 434 us, 32 x 752x480 2.36 / 2.40 ms, 8 x
+  // 1920x1080 6.64 / 8.04): all branches start together.  Results do not depend
+  // on it.
   void set_stagger(bool on) { stagger_ = on; }
   bool stagger() const { return stagger_; }
   int coarse_cells() const { return coarse_cells_; }
@@ -276,7 +267,7 @@ private:
   bool graphs_ = true;
   int parity_ = 0;
   size_t group_bytes_ = kDefaultGroupBytes;
-  int coarse_cells_ = QM_DEFAULT_COARSE_CELLS;
+  int coarse_cells_ = kCoarseAuto;
   int last_launches_ = 0;
   bool autotune_ = true;
   Tune fixed_tune_, last_tune_;

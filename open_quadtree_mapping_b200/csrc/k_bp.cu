@@ -1127,15 +1127,21 @@ bool coarse_plan(CoarsePlan &plan, int d, const long *cells, int levels, const i
   // of 512 / 8 of 512): 160x128 x 64, 8 streams 215 / 161 / 171 us, 12 225 / 172
   // / 181, 16 294 / 236 / 198; 320x240 8 267 / 255 / 272, 12 331 / 306 / 316;
   // 752x480 12 951 / 943 / 937, 24 1858 / 1809 / 1783.
-  for (int l = levels - 1; l >= 0 && iters[l] >= 2 && cells[l] <= max_cells; --l)
+  for (int l = levels - 1; l >= 0 && iters[l] >= 2; --l)
   {
     bool ok = false;
     by_d(d, [&](auto dc) {
       constexpr int D = decltype(dc)::value;
       const int wide = coarse_wide_d<D>(plan.keep != 0, arith);
+      // lane groups of a cluster x 2 colours x rounds
+      const long most = max_cells != kCoarseAuto ? max_cells
+                                                 : kCoarseMaxCtas * kCoarseMaxThreads /
+                                                       QuadLayout<D>::LPC * 2L *
+                                                       (jobs > 1 && jobs <= wide ? 2 : 1);
       const int first = jobs <= 2 * wide ? kCoarseMaxCtas : 8;
       for (int ctas : {first, kCoarseMaxCtas + 8 - first})
-        ok = ok || ((ctas <= 8 || wide > 0) && coarse_fit_d<D>(plan, cells[l], ctas, jobs > wide));
+        ok = ok || (cells[l] <= most && (ctas <= 8 || wide > 0) &&
+                    coarse_fit_d<D>(plan, cells[l], ctas, jobs > wide));
     });
     if (!ok)
       break;

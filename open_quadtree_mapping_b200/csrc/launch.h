@@ -145,6 +145,7 @@ void launch_bp_sweep_io(const Batch &B, int d, int level, int it, const SweepIO 
 // level in shared memory, `per` cells per block.
 constexpr int kCoarseMaxThreads = 1024;
 constexpr int kCoarseMaxCtas = 16; // above the portable 8: asked of the device
+constexpr int kCoarseAuto = -1; // max_cells of coarse_plan: by the half-sweeps' rounds
 struct CoarsePlan
 {
   int lo, hi;
@@ -158,6 +159,15 @@ struct CoarsePlan
 // branches running at once: the top levels with at most max_cells cells in every
 // job (cells[l]: the most), two half-sweeps or more, and room in a cluster's shared
 // memory.  False: no such level.  plan.keep is read, the rest (but hist) written.
+// kCoarseAuto takes the levels of whose cells a colour is one round of a full
+// cluster's lane groups, or two where a few streams run: above that a half-sweep in
+// the cluster takes longer than a launch over the whole GPU.  Measured (resident
+// pass, with the level in the cluster / launched, cells x lanes per cell in
+// brackets): one stream 320x240 x 64 (19200) 145 / 152 us, 752x480 x 64 (22560) 210 /
+// 212, 320x240 x 96 (38400) 175 / 164, 752x480 x 96 (45120) 256 / 236, 1280x720 x 64
+// (57600) 306 / 282; four (their launches are not early) 480x320 x 64 (38400) 233 /
+// 239, 1280x720 x 64 (57600) 654 / 675, 320x240 x 64 (76800) 187 / 169; 24 in
+// clusters of 8: 752x480 x 64 (22560) 1530 / 1539, 160x128 x 128 (40960) 302 / 241.
 bool coarse_plan(CoarsePlan &plan, int d, const long *cells, int levels, const int *iters,
                  long max_cells, int jobs, int arith);
 // jobs j0 .. j0 + jobs - 1 of the batch (B.jobs null: the inline job)
