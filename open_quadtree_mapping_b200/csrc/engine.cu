@@ -308,7 +308,8 @@ int enqueue_range(const Batch &B, const StageTable &T, const qm_params &p, size_
   });
   all(kFuseTransform, st.ftrans(),
       [&](const Batch &b, int g) { launch_fuse_transform(b, g, T.cuts.transform_px, ar, s); });
-  all(kFuseUpdate, st.fupd(), [&](const Batch &b, int g) { launch_fuse_update(b, g, T.cuts.update_px, s); });
+  all(kFuseUpdate, st.fupd(),
+      [&](const Batch &b, int g) { launch_fuse_update(b, g, T.cuts.update_px, s); });
   check(cudaGetLastError(), "kernel launch");
   return n;
 }

@@ -801,9 +801,8 @@ __device__ __forceinline__ void quad_argmin(const float (&b)[4], int gl, float &
 // Extraction, one lane group per level-0 cell, 16 bytes per lane and image as
 // in the half-sweeps (five images read, 4 bytes per leaf written).
 // Measured, one hypothesis every 8 to 32 per lane -> four consecutive ones:
-// 32 x 752x480 x 64 180 -> 152 us, 8 x 1920x1080 x 128 457 -> 316 us, with the
-// half-sweeps' memory rate reached at 128 hypotheses (5.1 GB at most, less the
-// cells that are no leaf origin).
+// 32 x 752x480 x 64 180 -> 152 us, 8 x 1920x1080 x 128 457 -> 316 us (2.65 GB if
+// every cell were a leaf origin; the others are not read).
 template <int D, int ARITH>
 __global__ void __launch_bounds__(kMaxCellWarps * 32)
     k_extract(const __grid_constant__ Batch B)
@@ -899,9 +898,11 @@ void sweep_d(const Batch &B, int blocks, int level, int parity, int first, int i
              KParams kp, int arith, int warps, cudaStream_t s)
 {
   if (arith == QM_ARITH_IEEE)
-    launch_kernel(k_bp_sweep<D, QM_ARITH_IEEE>, blocks, warps * 32, 0, s, B.early, B, level, parity, first, inherit, kp);
+    launch_kernel(k_bp_sweep<D, QM_ARITH_IEEE>, blocks, warps * 32, 0, s, B.early, B, level,
+                  parity, first, inherit, kp);
   else
-    launch_kernel(k_bp_sweep<D, QM_ARITH_REFERENCE>, blocks, warps * 32, 0, s, B.early, B, level, parity, first, inherit, kp);
+    launch_kernel(k_bp_sweep<D, QM_ARITH_REFERENCE>, blocks, warps * 32, 0, s, B.early, B, level,
+                  parity, first, inherit, kp);
 }
 
 // Opt-ins of one k_bp_coarse instance on the current device (large shared
@@ -1013,9 +1014,11 @@ void sweep_io_d(const Batch &B, int blocks, int level, int it, const SweepIO &io
                 int arith, cudaStream_t s)
 {
   if (arith == QM_ARITH_IEEE)
-    launch_kernel(k_bp_sweep_io<D, QM_ARITH_IEEE>, blocks, kCellWarps * 32, 0, s, B.early, B, level, it & 1, it == 0, io, kp);
+    launch_kernel(k_bp_sweep_io<D, QM_ARITH_IEEE>, blocks, kCellWarps * 32, 0, s, B.early, B,
+                  level, it & 1, it == 0, io, kp);
   else
-    launch_kernel(k_bp_sweep_io<D, QM_ARITH_REFERENCE>, blocks, kCellWarps * 32, 0, s, B.early, B, level, it & 1, it == 0, io, kp);
+    launch_kernel(k_bp_sweep_io<D, QM_ARITH_REFERENCE>, blocks, kCellWarps * 32, 0, s, B.early, B,
+                  level, it & 1, it == 0, io, kp);
 }
 
 template <int D>
@@ -1077,28 +1080,13 @@ void launch_msg_inherit(const Batch &B, int blocks, int level, int iters, int qt
 
 // A batch with mixed hypothesis counts launches one sweep per count present;
 // each launch skips the jobs of other counts.
-namespace
-{
-void sweep_any(const Batch &B, int blocks, int d, int level, int parity, int first, int inherit,
-               KParams kp, int arith, int warps, cudaStream_t s)
-{
-  switch (d)
-  {
-  case 32: sweep_d<32>(B, blocks, level, parity, first, inherit, kp, arith, warps, s); break;
-  case 48: sweep_d<48>(B, blocks, level, parity, first, inherit, kp, arith, warps, s); break;
-  case 64: sweep_d<64>(B, blocks, level, parity, first, inherit, kp, arith, warps, s); break;
-  case 96: sweep_d<96>(B, blocks, level, parity, first, inherit, kp, arith, warps, s); break;
-  case 128: sweep_d<128>(B, blocks, level, parity, first, inherit, kp, arith, warps, s); break;
-  default: break;
-  }
-}
-} // namespace
-
 void launch_bp_sweep(const Batch &B, int blocks, int d, int level, int it, KParams kp, int arith,
                      cudaStream_t s, int warps, int inherit)
 {
-  sweep_any(B, blocks, d, level, it & 1, it == 0 ? 1 : 0, inherit && it < 2 ? 1 : 0, kp, arith,
-            warps, s);
+  by_d(d, [&](auto dc) {
+    sweep_d<decltype(dc)::value>(B, blocks, level, it & 1, it == 0 ? 1 : 0,
+                                 inherit && it < 2 ? 1 : 0, kp, arith, warps, s);
+  });
 }
 
 void launch_bp_sweep_io(const Batch &B, int d, int level, int it, const SweepIO &io, KParams kp,

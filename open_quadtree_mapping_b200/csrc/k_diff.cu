@@ -26,9 +26,9 @@
 // (depth_upsample.cu:20-302) with every inner edge weight multiplied by a
 // per-pixel factor omega (the edge between a pixel and its left / upper
 // neighbour takes that pixel's factor), solved per line in FP64 by the Thomas
-// algorithm (its recurrences scanned by a warp per line).  The systems are symmetric, so the adjoint solve is the same
-// solve; dL/dw for the edge (k-1, k) is -lambda (g(k) - g(k-1)) (s(k) -
-// s(k-1)) summed over the two right-hand sides.
+// algorithm (its recurrences scanned by a warp per line).  The systems are
+// symmetric, so the adjoint solve is the same solve; dL/dw for the edge (k-1, k)
+// is -lambda (g(k) - g(k-1)) (s(k) - s(k-1)) summed over the two right-hand sides.
 //
 // Fusion adjoint: the update of fuse_currentmap evaluated on dual numbers
 // (value, derivative with respect to the upsampled depth).
@@ -1141,14 +1141,16 @@ template <int D, class R>
 void readout_d(const DiffBpR<R> &a, int backward, cudaStream_t s)
 {
   const int cells = a.w * a.h;
-  launch_kernel(k_soft_readout<D, R>, (cells + kDiffWarps - 1) / kDiffWarps, kDiffWarps * 32, 0, s, 1, a, backward);
+  launch_kernel(k_soft_readout<D, R>, (cells + kDiffWarps - 1) / kDiffWarps, kDiffWarps * 32, 0, s,
+                1, a, backward);
 }
 
 template <int D, class R>
 void bwd_d(const DiffBpR<R> &a, cudaStream_t s)
 {
   const int items = ((a.w + 1) / 2) * a.h;
-  launch_kernel(k_bp_sweep_bwd<D, R>, (items + kDiffWarps - 1) / kDiffWarps, kDiffWarps * 32, 0, s, 1, a);
+  launch_kernel(k_bp_sweep_bwd<D, R>, (items + kDiffWarps - 1) / kDiffWarps, kDiffWarps * 32, 0, s,
+                1, a);
 }
 
 template <class F>
@@ -1194,7 +1196,8 @@ void downsample(const DiffBpR<R> &a, const MsgPtrsR<R> &parent, int pw, int ph, 
 {
   const long n = (long)pw * ph * a.D;
   if (n > 0)
-    launch_kernel(k_msg_downsample<R>, (unsigned)((n + 255) / 256), 256, 0, s, 1, a, parent, pw, ph);
+    launch_kernel(k_msg_downsample<R>, (unsigned)((n + 255) / 256), 256, 0, s, 1, a, parent, pw,
+                  ph);
 }
 } // namespace
 
@@ -1277,7 +1280,8 @@ void upw_rows(const DiffUp &u, cudaStream_t s)
 {
   const int c = upw_lines(u.W, 2);
   if (c > 0)
-    launch_kernel(k_upw_rows<BWD>, (u.H + c - 1) / c, 32 * c, kUpwTableBytes + c * upw_line_doubles(u.W) * sizeof(double), s, 1, u);
+    launch_kernel(k_upw_rows<BWD>, (u.H + c - 1) / c, 32 * c,
+                  kUpwTableBytes + c * upw_line_doubles(u.W) * sizeof(double), s, 1, u);
   else if (BWD)
     k_upw_rows_bwd<<<(u.H + 63) / 64, 64, 0, s>>>(u);
   else
@@ -1289,7 +1293,8 @@ void upw_cols(const DiffUp &u, cudaStream_t s)
 {
   const int c = upw_lines(u.H, 4);
   if (c > 0)
-    launch_kernel(k_upw_cols<BWD>, (u.W + c - 1) / c, 32 * c, kUpwTableBytes + c * upw_line_doubles(u.H) * sizeof(double), s, 1, u);
+    launch_kernel(k_upw_cols<BWD>, (u.W + c - 1) / c, 32 * c,
+                  kUpwTableBytes + c * upw_line_doubles(u.H) * sizeof(double), s, 1, u);
   else if (BWD)
     k_upw_cols_bwd<<<(u.W + 63) / 64, 64, 0, s>>>(u);
   else

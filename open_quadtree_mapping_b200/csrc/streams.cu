@@ -230,7 +230,8 @@ void StreamSet::set_semidense(bool on)
     {
       check(cudaHostAlloc((void **)&h_sdjobs_[q], sizeof(SdJob) * n, cudaHostAllocDefault),
             "pinned allocation");
-      check(cudaHostAlloc((void **)&h_sdprefix_[q], sizeof(int) * 2 * (n + 1), cudaHostAllocDefault),
+      check(cudaHostAlloc((void **)&h_sdprefix_[q], sizeof(int) * 2 * (n + 1),
+                          cudaHostAllocDefault),
             "pinned allocation");
     }
     check(cudaMalloc((void **)&d_sdjobs_, sizeof(SdJob) * n), "device allocation");
