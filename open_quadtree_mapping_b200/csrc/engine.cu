@@ -1138,6 +1138,10 @@ void Engine::profile(const std::vector<int> &active, float *ms, int *launches)
   LaunchProfile prof;
   try
   {
+    // a first quadtree pass (it only repeats what it writes) keeps the GPU busy
+    // while the host enqueues: the first event pair would otherwise hold the
+    // launch's latency too
+    enqueue_range(B, pl.table(), params_, group_bytes_, coarse_cells_, st.qt(), st.qt(), stream_);
     enqueue_range(B, pl.table(), params_, group_bytes_, coarse_cells_, 0, st.count() - 1, stream_,
                   &prof);
     check(cudaStreamSynchronize(stream_), "profile run");
