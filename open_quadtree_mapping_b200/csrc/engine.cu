@@ -51,7 +51,10 @@ struct Stages
   int count() const { return 6 + 3 * L; }
 };
 
-// How the work of one launch is cut, by the size of all its jobs together.
+// How the work of one launch is cut, by the size of all streams that run together:
+// its branches are on the GPU at the same time (by a branch's own size instead: 2 to
+// 32 streams of 160x128 to 1920x1080 within 1 %, 16 of 160x128 4 % faster, 32 of
+// them 2 % slower).
 struct Cuts
 {
   int cost_split = 1;                   // blocks per tile of the cost kernel

@@ -75,8 +75,9 @@ __device__ __forceinline__ float mean_of(float sum)
 // does not have adds 0 there, which changes no sum.
 // Bound: launches where few streams run (a launch per level took three where one
 // does: 640x480 x 48 BP alone 126 -> 122 us, one 160x128 keyframe 189 -> 184 us),
-// DRAM where many do (the finest data term is read once: 32 x 752x480 x 64 82 us
-// both ways, the finest level's 185 MB are most of it).
+// DRAM where many do: 32 x 752x480 x 64 75 us, where a kernel per level took 64 in
+// three launches and the gaps between them (this one launched level by level: the
+// pass 2.38 ms instead of 2.35).
 __global__ void __launch_bounds__(kFlatThreads)
     k_pyramid(const __grid_constant__ Batch B, int level, int n)
 {
@@ -505,8 +506,8 @@ __global__ void __launch_bounds__(kMaxCellWarps * 32, 4)
 // trip counts depend only on the job and the plan.
 // Measured (the launch, one stream, messages through L2 with 8 blocks of 512
 // threads -> this one): 160x128 (34 half-sweeps) 113 -> 69 us, 752x480 (levels
-// 2 and 3) 99 -> 49, 1280x720 198 -> 79, 640x480 x 48 92 -> 47; clusters of 8
-// and 4 blocks: 752x480 76 and 105 us.
+// 2 and 3) 99 -> 49, 640x480 x 48 92 -> 47; clusters of 8 and 4 blocks: 752x480 76
+// and 105 us.  Which levels and how wide a cluster: coarse_plan.
 struct CoarseCell
 {
   unsigned short local, flags; // index in the block; CoarseFlag bits

@@ -206,7 +206,7 @@ constexpr int kCostWarps = kFlatThreads / 32;
 // values.  The balance depends on the hypothesis and slot counts, so the
 // engine's autotuner picks it per stream set.
 //
-// Bound: instruction issue (75 % busy; with nine byte gathers per node,
+// Bound: instruction issue (71 to 75 % busy; with nine byte gathers per node,
 // hypothesis and slot it was 133 instructions each, and L1 80 % busy).  Where
 // the patch is aligned (SlotParam) its three rows come as two aligned words each
 // and three byte-wise SADs, from one address; coordinates are packed pairs, and
@@ -215,9 +215,12 @@ constexpr int kCostWarps = kFlatThreads / 32;
 // position goes to the warp's list, and the list is worked off 32 at a time,
 // every lane busy.  Slots that turn further take every pixel at its own
 // position.  The sums are integers, so all ways give the same.  Measured, nine
-// gathers for every patch before: 32 x 752x480 x 64, 5 slots 0.838 -> 0.724 ms,
-// 8 x 1920x1080 x 128, 20 slots 4.93 -> 4.36, one 1280x720, 10 slots 0.144 ->
-// 0.123, one 1920x1080 x 128, 18 slots 0.870 -> 0.689.
+// gathers for every patch before, on views of which all patches are aligned (the
+// scenes of perf/cases.py): 32 x 752x480 x 64, 5 slots 0.838 -> 0.724 ms, 8 x
+// 1920x1080 x 128, 20 slots 4.93 -> 4.36, one 1280x720, 10 slots 0.144 -> 0.123,
+// one 1920x1080 x 128, 18 slots 0.870 -> 0.689.  The gain is the scene's: on
+// bench.py's views, which turn by 1 to 2 degrees a frame (94 to 97 % aligned), the
+// first is 0.881 -> 0.842 in eager launches, where the others' is 0.900 -> 0.752.
 // WORDS: the slot images' rows all start on a word, so that a patch's rows are
 // offset alike.  VIEW: the hypotheses out of a slot's view are found first
 // (kViewWork).

@@ -19,9 +19,12 @@ void check(cudaError_t e, const char *what);
 // set up while the kernel before it in the stream still runs, which hides the
 // launch's own latency.  For one stream's work or one keyframe's: with several
 // streams on the GPU the waiting blocks only take the others' place.  Measured,
-// late -> early: BP of one 640x480 x 48 keyframe (20 launches) 160 -> 128 us, a
+// late -> early: BP of one 640x480 x 48 keyframe (20 launches then) 160 -> 128 us, a
 // fitting step at 160x128 848 -> 765, a 160x128 stream (in its graph) 194 -> 190;
-// 32 x 752x480 (submit + wait) 3.19 -> 3.47 ms, so not there.
+// 32 x 752x480 (submit + wait) 3.19 -> 3.47 ms, so not there.  Several handles of one
+// stream each on threads are not told apart from one: a frame at 160x128 with 2 / 4 /
+// 8 of them 107 / 77 / 66 us late and 103 / 73 / 66 early, at 752x480 415 / 309 / 362
+// and 406 / 298 / 388 (runs of one kind differ by up to 15 %).
 template <class... P, class... A>
 void launch_kernel(void (*k)(P...), int blocks, int threads, size_t smem, cudaStream_t s,
                    int early, A &&...args)
