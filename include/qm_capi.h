@@ -188,7 +188,8 @@ int qm_batch_get_point_cloud(qm_batch *b, int stream, float *points, size_t capa
 int qm_batch_get_depths(qm_batch *b, int n, const int *streams, float *const *outs,
                         const size_t *strides);
 /* Re-runs the last dense pass of every stream on the frames already resident
- * on the device, also after frames that gave no result (no host transfers); used to time the device path alone. */
+ * on the device, also after frames that gave no result (no host transfers);
+ * used to time the device path alone. */
 int qm_batch_run_resident(qm_batch *b);
 /* Device pointer of stream i's fused depth map (row-major, dense). */
 int qm_batch_device_depth(qm_batch *b, int stream, const float **dev_ptr);
